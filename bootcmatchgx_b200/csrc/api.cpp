@@ -183,10 +183,24 @@ void choose_level_kernels(bcmgx_hierarchy* H)
         const bool f32 = p->vcycle_precision == BCMGX_VCYCLE_FP32 && l < L - 1;
         int code;
         if (!force.empty()) code = force[std::min(l, (int)force.size() - 1)];
-        else if (p->autotune) code = autotune_tpr(V, f32, H->stream);
+        else if (p->autotune) code = autotune_tpr(V, f32, l == 0 || !f32, H->stream);
         else code = default_tpr(V.A.n, V.A.nnz);
         // negative: the staged kernel with -code threads per row (1, 2, 4 or 8); kSlicedCode: the
         // sliced kernel (one lane per row: the CSR kernels stand in for it with 1 thread per row)
+        if (code == kStencilCode) {
+            build_stencil(V.A, l == 0 || !f32, H->stream);
+            V.A.stencil = V.A.st_form.p != nullptr;
+            if (V.A.stencil) {
+                release_sliced(V.A);
+                V.A.staged = false;
+                V.A.tpr = 1;
+                continue;
+            }
+            // a level that has no stencil form (a forced code, or a matrix of the same size as the one
+            // the code was tuned on): the sliced kernels, which take any level
+            code = kSlicedCode;
+        }
+        release_stencil(V.A);
         if (code == kSlicedCode) {
             build_sliced(V.A, H->stream);
             V.A.sliced = V.A.sl_ptr.p != nullptr;
@@ -596,8 +610,8 @@ int bcmgx_hierarchy_get_info(const bcmgx_hierarchy* h, bcmgx_hierarchy_info* inf
         for (int l = 0; l < info->num_levels && l < BCMGX_MAX_LEVELS; l++) {
             info->n[l] = h->lv[l].A.n;
             info->nnz[l] = h->lv[l].A.nnz;
-            info->tpr[l] = h->lv[l].A.sliced ? kSlicedCode : h->lv[l].A.staged ? -h->lv[l].A.tpr : h->lv[l].A.tpr;
-            info->index_bytes[l] = h->lv[l].A.sl_pid.p ? 0 : h->lv[l].A.dcol.p ? 2 : 4;
+            info->tpr[l] = h->lv[l].A.stencil ? kStencilCode : h->lv[l].A.sliced ? kSlicedCode : h->lv[l].A.staged ? -h->lv[l].A.tpr : h->lv[l].A.tpr;
+            info->index_bytes[l] = h->lv[l].A.sl_pid.p || h->lv[l].A.stencil ? 0 : h->lv[l].A.dcol.p ? 2 : 4;
             info->value_codes[l] = h->lv[l].A.vcode.p ? h->lv[l].A.nvalues : 0;
         }
         info->op_cmplx = h->op_cmplx;

@@ -138,6 +138,11 @@ struct DBuf {
     T* get() const { return p; }
 };
 
+// The stencil of a level in the stencil form (stencil.cuh): its column offsets, ascending.
+struct StencilOffs {
+    int o[32];
+};
+
 // Device CSR with an optional FP32 copy of the values (FP32 V-cycle).
 struct DevCsr {
     int n = 0, m = 0;
@@ -174,6 +179,18 @@ struct DevCsr {
     DBuf<unsigned char> sl_pid;
     DBuf<short> sl_pat;
     int npat = 0, patw = 0;
+    // stencil form (stencil.cuh, build_stencil), built when the level's tuning picks its kernels (tpr
+    // is then 1, as for the sliced ones): st_u offsets, st_nform forms (one byte per row, a mask of
+    // offsets each), and either the forms' values (st_tab64, and st_tab32 in an FP32 level) or every
+    // row's (st_val64 / st_val32, slices of 32 rows)
+    bool stencil = false;
+    StencilOffs st_offs {};
+    int st_u = 0, st_nform = 0;
+    int st_box = 0;   // line length of a 27-point box (stencil_box), 0: another stencil
+    DBuf<unsigned char> st_form;
+    DBuf<unsigned> st_mask;
+    DBuf<double> st_tab64, st_val64;
+    DBuf<float> st_tab32, st_val32;
 };
 
 // tuning code of the sliced kernels (hierarchy info, BCMGX_TPR, the tuning cache); the staged
@@ -185,6 +202,37 @@ void build_sliced(DevCsr& A, cudaStream_t s);
 // does not qualify. BCMGX_SLPAT=0 turns it off.
 void build_patterns(DevCsr& A, cudaStream_t s);
 void release_sliced(DevCsr& A);
+// Stencil form of a square level whose rows take their columns from at most 32 offsets and at most
+// 255 forms (three host round trips); leaves A.st_form empty when the level does not qualify.
+// need64: the FP64 values are wanted too (always when the level has no FP32 ones). BCMGX_STENCIL=0
+// turns it off.
+constexpr int kStencilCode = 65;
+// Line length s of the 27 offsets pl[a] + (b - 1) s + (c - 1) of a box (three planes, pl[1] = 0), else 0.
+inline int stencil_box(int u, const StencilOffs& so)
+{
+    if (u != 27) return 0;
+    const int s = so.o[4] - so.o[1];
+    for (int k = 0; k < 27; k++)
+        if (so.o[k] != so.o[9 * (k / 9) + 4] + (k / 3 % 3 - 1) * s + (k % 3 - 1)) return 0;
+    return so.o[13] == 0 ? s : 0;
+}
+// blocks of 4 offsets that the stencil kernels are compiled for: the least of these with room for u
+inline int stencil_blocks(int u) { return u <= 8 ? 2 : u <= 16 ? 4 : u <= 28 ? 7 : 8; }
+void build_stencil(DevCsr& A, bool need64, cudaStream_t s);
+void release_stencil(DevCsr& A);
+
+// A small level's sweep chains as one cluster launch (chain.cu): ctas blocks of R rows, the level's
+// entries by block and slice, the lists of values that blocks exchange, the shared-memory layout.
+struct ChainPlan {
+    int ctas = 0, n = 0, R = 0, S = 0, ns = 0, st = 0, ecap = 0, scap = 0;
+    bool f32 = false;
+    size_t smem = 0;
+    int off_f = 0, off_M = 0, off_x1 = 0, off_val = -1, off_idx = -1;
+    DBuf<unsigned char> val;
+    DBuf<unsigned short> idx;
+    DBuf<unsigned> push;
+    DBuf<int> sptr, sizes;
+};
 
 struct Level {
     DevCsr A;
@@ -438,7 +486,9 @@ inline void ensure_smem_limit(void (*kernel)(A...), size_t bytes)
 }
 
 // ---- kernels usable on raw device memory (kernels.cu) ----
-int autotune_tpr(Level& V, bool f32, cudaStream_t s);
+constexpr int kTuneMinRows = 20000;   // rows of the smallest level that the autotuner times
+// need64: see build_stencil
+int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s);
 void choose_level_kernels(bcmgx_hierarchy* H);
 void stage_fault_init();
 void stage_fault_check();

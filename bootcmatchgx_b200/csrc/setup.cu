@@ -2199,6 +2199,191 @@ void finish_level_matrix(Level& V, bool want_f32, cudaStream_t s)
     const int n = V.A.n;
     build_offsets(V.A, s);
     V.M.alloc(n, s);
+// ---- stencil form ------------------------------------------------------------------------------
+// Hashes of every row's offsets (ho) and of its offsets and values (hf), 63 bits each.
+__global__ void k_st_hash(int n, const int* __restrict__ row, const int* __restrict__ col, const double* __restrict__ val,
+    unsigned long long* __restrict__ ho, unsigned long long* __restrict__ hf)
+{
+    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
+        const int b = row[r], e = row[r + 1];
+        unsigned long long o = 1469598103934665603ull ^ (unsigned long long)(e - b), w = o;
+        for (int j = b; j < e; j++) {
+            const unsigned long long d = (unsigned)(col[j] - (int)r);
+            // the values' low bits are often all zero: fold the high ones down first
+            unsigned long long v = (unsigned long long)__double_as_longlong(val[j]);
+            v = (v ^ (v >> 32)) * 0x9E3779B97F4A7C15ull;
+            v ^= v >> 29;
+            o = (o ^ d) * 1099511628211ull;
+            w = ((w ^ d) * 1099511628211ull ^ v) * 1099511628211ull;
+        }
+        ho[r] = o & 0x7fffffffffffffffull;   // never kVcEmpty
+        hf[r] = w & 0x7fffffffffffffffull;
+    }
+}
+
+// offs[id * 32 + k], vals[id * 32 + k]: entry k of form id's representative row; len[id] its length
+__global__ void k_st_forms(int nform, const int* __restrict__ row, const int* __restrict__ col,
+    const double* __restrict__ val, const int* __restrict__ rep, const int* __restrict__ len, int* __restrict__ offs,
+    double* __restrict__ vals)
+{
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nform * 32; t += gridDim.x * blockDim.x) {
+        const int id = t >> 5, k = t & 31, r = rep[id];
+        const bool in = r >= 0 && k < len[id];
+        offs[t] = in ? col[row[r] + k] - r : 0;
+        vals[t] = in ? val[row[r] + k] : 0.0;
+    }
+}
+
+// Checks every row against its form (a hash collision must not stand): the offsets the form's mask
+// names, and with the table (tab, up values a form) the values' bits. Without it the row's values
+// are written to their slots (v64, v32; rows past n are zero).
+__global__ void k_st_fill(int n, long total, int u, StencilOffs so, const int* __restrict__ row,
+    const int* __restrict__ col, const double* __restrict__ val, const unsigned char* __restrict__ form,
+    const unsigned* __restrict__ mask, const double* __restrict__ tab, int up, double* __restrict__ v64,
+    float* __restrict__ v32, int* bad)
+{
+    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < total; r += (long)gridDim.x * blockDim.x) {
+        const bool live = r < n;
+        int j = live ? row[r] : 0;
+        const int e = live ? row[r + 1] : 0;
+        const int id = live ? form[r] : 0;
+        const unsigned m = live ? mask[id] : 0u;
+        bool ok = !live || __popc(m) == e - j;
+        for (int k = 0; k < u; k++) {
+            double v = 0.0;
+            if (ok && ((m >> k) & 1u)) {
+                v = val[j];
+                ok = col[j] == (int)r + so.o[k] &&
+                    (!tab || __double_as_longlong(v) == __double_as_longlong(tab[(long)id * up + k]));
+                j++;
+            }
+            if (v64) v64[(r >> 5) * (32L * u) + 32 * k + (r & 31)] = v;
+            if (v32) v32[(r >> 5) * (32L * u) + 32 * k + (r & 31)] = (float)v;
+        }
+        if (!ok) atomicOr(bad, 1);
+    }
+}
+
+void build_stencil(DevCsr& A, bool need64, cudaStream_t s)
+{
+    if (A.st_form.p) return;
+    const char* env = std::getenv("BCMGX_STENCIL");
+    if (env && env[0] == '0') return;
+    const int n = A.n;
+    if (n <= 0 || A.m != n || A.max_row <= 0 || A.max_row > 32) return;
+    const bool f32 = A.val32.p != nullptr;
+    DBuf<unsigned long long> ho, hf, keys;
+    DBuf<int> cnt;
+    ho.alloc(n, s);
+    hf.alloc(n, s);
+    keys.alloc(2 * kVcSlots, s);
+    cnt.alloc(4, s);
+    BCMGX_CUDA(cudaMemsetAsync(keys.p, 0xff, sizeof(unsigned long long) * 2 * kVcSlots, s));
+    BCMGX_CUDA(cudaMemsetAsync(cnt.p, 0, 4 * sizeof(int), s));
+    note_launch(); k_st_hash<<<gs_grid(n), 256, 0, s>>>(n, A.row.p, A.col.p, A.val.p, ho.p, hf.p);
+    note_launch(); k_vc_collect<<<gs_grid(n), 256, 0, s>>>(n, (const double*)hf.p, keys.p, cnt.p, cnt.p + 1);
+    note_launch(); k_vc_collect<<<gs_grid(n), 256, 0, s>>>(n, (const double*)ho.p, keys.p + kVcSlots, cnt.p + 2, cnt.p + 3);
+    BCMGX_CHECK_LAUNCH();
+    std::vector<unsigned long long> hk(2 * kVcSlots);
+    int hc[4] = { 0, 0, 0, 0 };
+    BCMGX_CUDA(cudaMemcpyAsync(hk.data(), keys.p, sizeof(unsigned long long) * 2 * kVcSlots, cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaMemcpyAsync(hc, cnt.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaStreamSynchronize(s));
+    int which = -1;   // 0: forms of offsets and values, 1: of offsets
+    for (int w = 0; w < 2 && which < 0; w++)
+        if (!hc[2 * w + 1] && hc[2 * w] > 0 && hc[2 * w] <= 255) which = w;
+    if (which < 0) return;
+    const unsigned long long* key = hk.data() + which * kVcSlots;
+    std::vector<unsigned long long> forms;
+    for (int t = 0; t < kVcSlots; t++)
+        if (key[t] != kVcEmpty) forms.push_back(key[t]);
+    std::sort(forms.begin(), forms.end());
+    const int nform = (int)forms.size();
+    std::vector<int> slot_id(kVcSlots, 0);
+    for (int t = 0; t < kVcSlots; t++)
+        if (key[t] != kVcEmpty) slot_id[t] = (int)(std::lower_bound(forms.begin(), forms.end(), key[t]) - forms.begin());
+    DBuf<int> sid, rep, len, foffs, bad;
+    DBuf<double> fvals;
+    DBuf<unsigned char> form;
+    sid.alloc(kVcSlots, s);
+    rep.alloc(nform, s);
+    len.alloc(nform, s);
+    foffs.alloc(nform * 32, s);
+    fvals.alloc(nform * 32, s);
+    bad.alloc(1, s);
+    form.alloc(n, s);
+    BCMGX_CUDA(cudaMemcpyAsync(sid.p, slot_id.data(), sizeof(int) * kVcSlots, cudaMemcpyHostToDevice, s));
+    BCMGX_CUDA(cudaMemsetAsync(rep.p, 0xff, sizeof(int) * nform, s));
+    BCMGX_CUDA(cudaMemsetAsync(len.p, 0, sizeof(int) * nform, s));
+    BCMGX_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
+    const double* hsel = (const double*)(which == 0 ? hf.p : ho.p);
+    note_launch(); k_vc_encode<<<gs_grid(n), 256, 0, s>>>(n, hsel, keys.p + which * kVcSlots, sid.p, form.p);
+    note_launch(); k_pat_rep<<<gs_grid(n), 256, 0, s>>>(n, A.row.p, form.p, rep.p, len.p);
+    note_launch(); k_st_forms<<<gs_grid(nform * 32), 256, 0, s>>>(nform, A.row.p, A.col.p, A.val.p, rep.p, len.p, foffs.p, fvals.p);
+    BCMGX_CHECK_LAUNCH();
+    std::vector<int> ho_offs(nform * 32), ho_len(nform);
+    std::vector<double> ho_vals(nform * 32);
+    BCMGX_CUDA(cudaMemcpyAsync(ho_offs.data(), foffs.p, sizeof(int) * nform * 32, cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaMemcpyAsync(ho_vals.data(), fvals.p, sizeof(double) * nform * 32, cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaMemcpyAsync(ho_len.data(), len.p, sizeof(int) * nform, cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaStreamSynchronize(s));
+    // the stencil: the union of the forms' offsets, ascending
+    std::vector<int> offs;
+    for (int id = 0; id < nform; id++) {
+        for (int k = 0; k < ho_len[id]; k++) offs.push_back(ho_offs[id * 32 + k]);
+        std::sort(offs.begin(), offs.end());
+        offs.erase(std::unique(offs.begin(), offs.end()), offs.end());
+        if (offs.size() > 32) return;
+    }
+    const int u = (int)offs.size();
+    if (u == 0) return;
+    // stored values take a slot for every row and offset: not worth it on a level that leaves a
+    // quarter of them empty (the slots then cost what the columns would)
+    if (which == 1 && 4 * A.nnz < 3 * (int64_t)u * n) return;
+    const int up = 4 * stencil_blocks(u);
+    std::vector<unsigned> mask(nform, 0u);
+    std::vector<double> t64((size_t)nform * up, 0.0);
+    std::vector<float> t32((size_t)nform * up, 0.0f);
+    for (int id = 0; id < nform; id++)
+        for (int k = 0; k < ho_len[id]; k++) {
+            const int q = (int)(std::lower_bound(offs.begin(), offs.end(), ho_offs[id * 32 + k]) - offs.begin());
+            mask[id] |= 1u << q;
+            t64[(size_t)id * up + q] = ho_vals[id * 32 + k];
+            t32[(size_t)id * up + q] = (float)ho_vals[id * 32 + k];
+        }
+    StencilOffs so {};
+    for (int k = 0; k < u; k++) so.o[k] = offs[k];
+    const long total = ((long)n + 31) / 32 * 32;   // whole 32-row slices
+    A.st_mask.alloc(nform, s);
+    BCMGX_CUDA(cudaMemcpyAsync(A.st_mask.p, mask.data(), sizeof(unsigned) * nform, cudaMemcpyHostToDevice, s));
+    if (which == 0) {
+        A.st_tab64.alloc(t64.size(), s);
+        BCMGX_CUDA(cudaMemcpyAsync(A.st_tab64.p, t64.data(), sizeof(double) * t64.size(), cudaMemcpyHostToDevice, s));
+        if (f32) {
+            A.st_tab32.alloc(t32.size(), s);
+            BCMGX_CUDA(cudaMemcpyAsync(A.st_tab32.p, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice, s));
+        }
+    } else {
+        if (need64 || !f32) A.st_val64.alloc((size_t)total * u, s);
+        if (f32) A.st_val32.alloc((size_t)total * u, s);
+    }
+    note_launch();
+    k_st_fill<<<gs_grid(total), 256, 0, s>>>(n, total, u, so, A.row.p, A.col.p, A.val.p, form.p, A.st_mask.p, A.st_tab64.p,
+        up, A.st_val64.p, A.st_val32.p, bad.p);
+    BCMGX_CHECK_LAUNCH();
+    // the host vectors above are read by their copies, and the form is complete (its kernels read it
+    // before their dependency wait), before this returns
+    if (read_err(bad.p, s)) {
+        release_stencil(A);
+        return;
+    }
+    A.st_form = std::move(form);
+    A.st_offs = so;
+    A.st_u = u;
+    A.st_nform = nform;
+    A.st_box = stencil_box(u, so);
+}
+
     if (want_f32) V.M32.alloc(n, s);
     note_launch(); k_abs_row_sum<<<gs_grid(n), 256, 0, s>>>(n, V.A.row.p, V.A.val.p, V.M.p, want_f32 ? V.M32.p : nullptr);
     if (want_f32) {

@@ -16,6 +16,7 @@
 #include "rowops.cuh"
 #include "staged.cuh"
 #include "sliced.cuh"
+#include "stencil.cuh"
 #include "blockops.cuh"
 #include "persist.cuh"
 
@@ -243,6 +244,18 @@ void release_sliced(DevCsr& A)
     A.sl_val64.release();
 }
 
+void release_stencil(DevCsr& A)
+{
+    A.stencil = false;
+    A.st_u = A.st_nform = A.st_box = 0;
+    A.st_form.release();
+    A.st_mask.release();
+    A.st_tab64.release();
+    A.st_val64.release();
+    A.st_tab32.release();
+    A.st_val32.release();
+}
+
 // Builds A's sliced copy from its CSR arrays (one host round trip for the total). The codes are
 // used when the level is coded and its table has a free (zero) slot for the padding.
 void build_sliced(DevCsr& A, cudaStream_t s)
@@ -322,6 +335,61 @@ static void launch_sliced(const DevCsr& A, SlSrc<VS> sv, const XT* x, const FT* 
     BCMGX_CHECK_LAUNCH();
 }
 
+// Rows per lane of the 27-point box kernel on a level (1: the general stencil kernel). More rows a
+// lane load less of x, but leave fewer warps: measured with 1 / 2 / 4 rows, FP32 sweeps take 47.6 / 28.5
+// / 26.8 us at 4.1 M rows, 12.2 / 9.7 / 10.1 at 1 M, 6.4 / 4.4 / 5.3 at 262 k, 3.9 / 3.6 / 4.2 at 125 k;
+// FP32 residuals 44.2 / 28.7 / 22.2, 11.3 / 9.0 / 8.6, 5.8 / 4.8 / 4.1, 3.9 / 3.4 / 3.6; FP64 sweeps 16.0 /
+// 15.1 / 16.5 at 1 M (the product and dots 79.0 / 62.1 / 64.3 at 4.1 M), 15.6 / 14.5 / 12.9 at 886 k, 6.6 /
+// 7.3 / 6.1 at 262 k, 4.3 / 5.4 / 5.1 at 125 k.
+static int box_rows(const DevCsr& A, int op, size_t xbytes)
+{
+    if (A.st_box <= 0 || A.n < 200000) return 1;
+    if (xbytes == 8) return A.n < 950000 ? 4 : 2;
+    return op == OP_RESID || A.n >= 2000000 ? 4 : 2;
+}
+
+template <int OP, bool TAB, typename VT, typename XT, typename FT, typename MT, typename YT>
+static void launch_stencil(const DevCsr& A, const VT* vals, const XT* x, const FT* f, const MT* M, YT* y, double alpha,
+    double beta, const int* skip, cudaStream_t s)
+{
+    if constexpr (TAB) {
+        const int P = box_rows(A, OP, sizeof(XT));
+        if (P > 1) {
+            const int bs = A.st_box;
+            const size_t smem = (size_t)A.st_nform * 36 * sizeof(VT);
+            const long items = ((long)A.n + (long)P * bs - 1) / ((long)P * bs) * bs;
+            auto go = [&](auto kern) {
+                ensure_smem_limit((const void*)kern, smem);
+                const int per_sm = blocks_per_sm((const void*)kern, kStThreads, smem);
+                const int grid = (int)std::max<long>(1, std::min<long>(ceil_div(items, kStThreads), (long)per_sm * num_sms()));
+                launch_dep<0>(kern, grid, kStThreads, smem, s, A.n, bs, A.st_offs.o[4], A.st_offs.o[22],
+                    (const unsigned char*)A.st_form.p, (const unsigned*)A.st_mask.p, A.st_nform, vals, x, f, M, y, alpha,
+                    beta, skip);
+                BCMGX_CHECK_LAUNCH();
+            };
+            if (P == 4) go(k_rowop_box27<OP, 4, VT, XT, FT, MT, YT>);
+            else go(k_rowop_box27<OP, 2, VT, XT, FT, MT, YT>);
+            return;
+        }
+    }
+    const int nb = stencil_blocks(A.st_u);
+    const size_t smem = TAB ? (size_t)A.st_nform * 4 * nb * sizeof(VT) : 0;
+    auto go = [&](auto kern) {
+        ensure_smem_limit((const void*)kern, smem);
+        const int per_sm = blocks_per_sm((const void*)kern, kStThreads, smem);
+        const int grid = (int)std::max<long>(1, std::min<long>(ceil_div(A.n, kStThreads), (long)per_sm * num_sms()));
+        launch_dep<0>(kern, grid, kStThreads, smem, s, A.n, A.st_u, A.st_offs, (const unsigned char*)A.st_form.p,
+            (const unsigned*)A.st_mask.p, A.st_nform, vals, x, f, M, y, alpha, beta, skip);
+        BCMGX_CHECK_LAUNCH();
+    };
+    switch (nb) {
+    case 2: go(k_rowop_stencil<OP, 2, TAB, VT, XT, FT, MT, YT>); break;
+    case 4: go(k_rowop_stencil<OP, 4, TAB, VT, XT, FT, MT, YT>); break;
+    case 7: go(k_rowop_stencil<OP, 7, TAB, VT, XT, FT, MT, YT>); break;
+    default: go(k_rowop_stencil<OP, 8, TAB, VT, XT, FT, MT, YT>); break;
+    }
+}
+
 // The row operation on a level matrix, through its int16 column offsets when it has them, through
 // its value codes when it has them and `val` is the level's own FP64 or FP32 value array (the
 // codes index a table of those same values), and through the staged kernel when the level's
@@ -351,7 +419,8 @@ static void launch_rowop_vs(int tpr, const DevCsr& A, VS val, const void* val_pt
 }
 
 // form (stage): -1 the level's tuned kernel (sliced, staged or plain), 0 the plain CSR kernel, 1 the
-// staged kernel, 2 the sliced kernel. The sliced kernel runs when the level has its sliced copy
+// staged kernel, 2 the sliced kernel, 3 the stencil kernel. The stencil kernel runs when the level
+// has its stencil form in the precision of `val`, the sliced kernel runs when the level has its sliced copy
 // and `val` is one of the level's own value arrays (else the CSR kernels do, with tpr).
 template <int OP, typename VT, typename XT, typename FT, typename MT, typename YT>
 static void launch_rowop_A(int tpr, const DevCsr& A, const VT* val, const XT* x, const FT* f, const MT* M, YT* y,
@@ -361,7 +430,10 @@ static void launch_rowop_A(int tpr, const DevCsr& A, const VT* val, const XT* x,
     const VT* own = nullptr;
     const VT* tab = nullptr;
     const VT* slv = nullptr;
+    const VT *stab = nullptr, *stv = nullptr;
     if constexpr (std::is_same<VT, float>::value) {
+        stab = A.st_tab32.p;
+        stv = A.st_val32.p;
         own = A.val32.p;
         tab = A.vtab32.p;
         slv = A.sl_val32.p;
@@ -369,6 +441,18 @@ static void launch_rowop_A(int tpr, const DevCsr& A, const VT* val, const XT* x,
         own = A.val.p;
         tab = A.vtab64.p;
         slv = A.sl_val64.p;
+        stab = A.st_tab64.p;
+        stv = A.st_val64.p;
+    }
+    if ((stage == 3 || (stage < 0 && A.stencil)) && A.st_form.p && val == own) {
+        if (stab) {
+            launch_stencil<OP, true>(A, stab, x, f, M, y, alpha, beta, skip, s);
+            return;
+        }
+        if (stv) {
+            launch_stencil<OP, false>(A, stv, x, f, M, y, alpha, beta, skip, s);
+            return;
+        }
     }
     if ((stage == 2 || (stage < 0 && A.sliced)) && A.sl_ptr.p && val == own) {
         if (A.sl_code.p && tab) {
@@ -1452,8 +1536,8 @@ __global__ void __launch_bounds__(kRedThreads) k_fcg_norm0(int n, const double* 
 
 static void fcg_resid0(const DevCsr& A, const double* x, const double* b, double* r, FcgState* st, double* part, cudaStream_t s)
 {
-    if (A.sliced) {
-        // the sliced kernel forms r = b - A x with the one-thread-per-row kernel's row sums; the
+    if (A.sliced || A.stencil) {
+        // the sliced and stencil kernels form r = b - A x with the one-thread-per-row kernel's row sums; the
         // norm follows in a kernel of its own
         rowop_resid(A, x, b, r, nullptr, s);
         auto k = k_fcg_norm0;
@@ -1750,7 +1834,6 @@ void time_block_kernels(bcmgx_hierarchy* H, int K, int reps, double* out)
 // matrices reuse them; when the environment variable BCMGX_TUNE_CACHE names a file, the cache is
 // also read from it at the first use and every new result is appended to it (one "rows nnz
 // precision code" line each).
-constexpr int kTuneMinRows = 20000;
 static std::mutex g_tune_mu;
 static std::map<std::tuple<int, int64_t, int>, int> g_tune_cache;
 static bool g_tune_loaded = false;
@@ -1767,7 +1850,7 @@ static void tune_cache_load()
     int n, prec, t;
     while (std::fscanf(f, "%d %lld %d %d", &n, &z, &prec, &t) == 4)
         if (t == 1 || t == 2 || t == 4 || t == 8 || t == 16 || t == 32 || t == -1 || t == -2 || t == -4 || t == -8 ||
-            t == kSlicedCode)
+            t == kSlicedCode || t == kStencilCode)
             g_tune_cache[std::make_tuple(n, (int64_t)z, prec)] = t;
     std::fclose(f);
 }
@@ -1782,12 +1865,13 @@ static void tune_cache_store(const std::tuple<int, int64_t, int>& key, int t)
     std::fclose(f);
 }
 
-int autotune_tpr(Level& V, bool f32, cudaStream_t s)
+int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
 {
     DevCsr& A = V.A;
     const int n = A.n;
     if (n < kTuneMinRows) return default_tpr(n, A.nnz);
-    const auto key = std::make_tuple(n, A.nnz, f32 ? 1 : 0);
+    // coded levels are tuned apart: a matrix of the same size with other values has other kernels
+    const auto key = std::make_tuple(n, A.nnz, (f32 ? 1 : 0) | (A.vcode.p ? 2 : 0));
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         tune_cache_load();
@@ -1817,9 +1901,12 @@ int autotune_tpr(Level& V, bool f32, cudaStream_t s)
     // candidates: 1..16 threads per row, the staged kernel with 1, 2, 4 and 8 (coded negative),
     // and the sliced kernel (its copy of the matrix is built for the trial and kept if it wins)
     build_sliced(A, s);
-    for (int t : {1, 2, 4, 8, 16, -1, -2, -4, -8, kSlicedCode}) {
+    build_stencil(A, need64, s);
+    for (int t : {1, 2, 4, 8, 16, -1, -2, -4, -8, kSlicedCode, kStencilCode}) {
         if (t == kSlicedCode && !A.sl_ptr.p) continue;
-        const int tp = t == kSlicedCode ? 1 : t < 0 ? -t : t, stage = t == kSlicedCode ? 2 : t < 0 ? 1 : 0;
+        if (t == kStencilCode && !A.st_form.p) continue;
+        const bool own = t == kSlicedCode || t == kStencilCode;
+        const int tp = own ? 1 : t < 0 ? -t : t, stage = t == kStencilCode ? 3 : t == kSlicedCode ? 2 : t < 0 ? 1 : 0;
         auto launch = [&] {
             if (f32)
                 launch_rowop_A<OP_JACOBI>(tp, A, A.val32.p, (const float*)a32.p, (const float*)c32.p, V.M32.p, b32.p, 1.0, 0.0, nullptr, s, stage);
@@ -1853,6 +1940,7 @@ int autotune_tpr(Level& V, bool f32, cudaStream_t s)
 template <int S>
 __global__ void __launch_bounds__(256) k_grad_pattern(int n, const int* __restrict__ row, const int* __restrict__ col,
     const double* __restrict__ lam, const double* __restrict__ x, double* __restrict__ dA)
+    if (best != kStencilCode) release_stencil(A);
 {
     const int lane = threadIdx.x & (S - 1);
     const long stride = (long)gridDim.x * blockDim.x / S;
@@ -2023,7 +2111,7 @@ struct BatchCaptureMode {
     {
         H->chain_in_block = true;
         for (Level& V : H->lv) {
-            staged.push_back((V.A.staged ? 1 : 0) | (V.A.sliced ? 2 : 0));
+            staged.push_back((V.A.staged ? 1 : 0) | (V.A.sliced ? 2 : 0) | (V.A.stencil ? 4 : 0));
             V.A.staged = false;
             V.A.sliced = false;
         }
@@ -2037,6 +2125,7 @@ struct BatchCaptureMode {
         }
     }
 };
+            V.A.stencil = false;
 
 void batch_build(bcmgx_batch* B)
 {
@@ -2046,6 +2135,7 @@ void batch_build(bcmgx_batch* B)
         ensure_solve_workspace(H);
         BatchCaptureMode mode(H);
         add_solve_to_graph(H, g);
+            H->lv[l].A.stencil = (staged[l] & 4) != 0;
     }
     BCMGX_CUDA(cudaGraphInstantiate(&B->exec, g, 0));
     BCMGX_CUDA(cudaGraphDestroy(g));
