@@ -778,11 +778,11 @@ int bcmgx_suitor_matching(int n, int64_t nnz, const int* row, const int* col, co
     return guarded([&] {
         BCMGX_REQUIRE(n > 0 && nnz > 0 && row && col && W && M, BCMGX_ERR_INVALID_INPUT, "bad argument");
         cudaStream_t s = (cudaStream_t)stream;
-        validate_csr_dev(n, n, nnz, row, col, false, s);
+        const int max_row = validate_csr_dev(n, n, nnz, row, col, false, s);
         DBuf<int> tpos;
         tpos.alloc(nnz, s);
         tpos_dev(n, nnz, row, col, tpos.p, s);
-        suitor_dev(n, nnz, row, col, W, tpos.p, M, 0, s);
+        suitor_dev(n, nnz, row, col, W, tpos.p, M, max_row, s);
         BCMGX_CUDA(cudaStreamSynchronize(s));
     });
 }

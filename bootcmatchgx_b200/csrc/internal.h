@@ -497,7 +497,8 @@ void launch_spmv(int n, const int* row, const int* col, const double* val, const
     double alpha, double beta, int tpr, cudaStream_t s);
 void edge_weights_dev(int n, int64_t nnz, const int* row, const int* col, const double* val,
     const double* w, double* W, int* tpos, double* min_out_host, cudaStream_t s);
-void validate_csr_dev(int n, int m, int64_t nnz, const int* row, const int* col, bool need_diag, cudaStream_t s);
+// Throws BCMGX_ERR_INVALID_INPUT for a malformed matrix; returns its longest row.
+int validate_csr_dev(int n, int m, int64_t nnz, const int* row, const int* col, bool need_diag, cudaStream_t s);
 void tpos_dev(int n, int64_t nnz, const int* row, const int* col, int* tpos, cudaStream_t s);
 // The edge weights formed inside the rank kernel (rows of at most 32 entries): the inputs of
 // k_logw's expression instead of the stored weights.

@@ -211,105 +211,107 @@ void scan_exclusive_dev(const int* in, int* out, long n, cudaStream_t s)
 // ------------------------------------------------------------------------------------------
 // matrix checks and small per-row kernels
 // ------------------------------------------------------------------------------------------
-__global__ void k_validate(int n, int m, long long nnz, const int* __restrict__ row, const int* __restrict__ col,
-    int* err, int* max_row, int need_diag)
-{
-    const int lane = threadIdx.x & 31;
-    int mx = 0;
-    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32; r < n; r += (long)gridDim.x * blockDim.x / 32) {
-        const int b = row[r], e = row[r + 1];
-        int bad = 0;
-        if (r == 0 && b != 0) bad |= ERR_ROW0;
-        if (r == n - 1 && (long long)e != nnz) bad |= ERR_ROWN;
-        if (e < b || b < 0 || (long long)e > nnz) {
-            bad |= ERR_ROWORDER;
-        } else {
-            bool diag = false;
-            for (int j = b + lane; j < e; j += 32) {
-                const int c = col[j];
-                if (c < 0 || c >= m) bad |= ERR_COLRANGE;
-                if (j > b && col[j - 1] >= c) bad |= ERR_COLSORT;
-                if (c == r) diag = true;
-            }
-            diag = __any_sync(0xffffffffu, diag);
-            if (need_diag && !diag) bad |= ERR_NODIAG;
-            mx = max(mx, e - b);
-        }
-        bad = __reduce_or_sync(0xffffffffu, bad);
-        if (lane == 0 && bad) atomicOr(err, bad);
-    }
-    if (lane == 0 && mx > 0) atomicMax(max_row, mx);
-}
+// Input checks of a CSR matrix: row offsets (0 at the start, not decreasing, nnz at the end), columns
+// in range and strictly ascending, and with need_diag a diagonal entry in every row; the longest row
+// goes to *max_row. OFFS: also the largest |col - row| to *max_off, the diagonal's position in every
+// row to dpos (-1: none) and, when dcol is given, every column as an int16 offset from its row
+// (clamped; the caller keeps them only when the largest offset fits).
+// A block takes 256 consecutive rows: their columns, one contiguous range, go to shared memory with
+// asynchronous copies that are all in flight at once, then every lane walks its own row there, one
+// word in 32 skipped so that rows of 32 entries do not meet in one bank. The pass is then bound by
+// the column stream: on the 27-point 160^3 matrix (437 MB of columns) the checked product takes 415 us
+// instead of 910, 236 of them the product, where a warp per row took 655 us for the checks. Rows whose block holds more
+// than kValCap entries, or an offset out of order, are walked by a warp each from global memory.
+constexpr int kValRows = 256;
+constexpr int kValCap = 8192;
 
-// The input checks of k_validate with 8 lanes per row (4 rows of a warp in flight, the previous
-// column passed by shuffles), plus the largest |col - row| and, when dcol is given, every column
-// as an int16 offset from its row (clamped; the caller keeps them only when the largest offset
-// fits): one pass over the input instead of three.
-__global__ void k_validate_offsets(int n, int m, long long nnz, const int* __restrict__ row, const int* __restrict__ col,
-    int* err, int* max_row, int* max_off, short* __restrict__ dcol, int need_diag, int* __restrict__ dpos)
+__device__ __forceinline__ int val_slot(int j) { return j + (j >> 5); }
+
+template <bool OFFS>
+__global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long nnz, const int* __restrict__ row,
+    const int* __restrict__ col, int* err, int* max_row, int* max_off, short* __restrict__ dcol, int need_diag,
+    int* __restrict__ dpos)
 {
-    constexpr int S = 8;
-    const int lane = threadIdx.x & (S - 1);
-    const int sub = (threadIdx.x & 31) / S;
-    const unsigned mask = 0xffu << (sub * S);
-    const long stride = (long)gridDim.x * blockDim.x / S;
-    int mx = 0, mo = 0;
-    for (long base = ((long)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / S; base < n; base += stride) {
-        const long r = base + sub;
-        int bad = 0;
-        if (r < n) {
-            const int b = row[r], e = row[r + 1];
+    __shared__ int rows_s[kValRows + 1];
+    __shared__ int cols_s[kValCap + kValCap / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    int mx = 0, mo = 0, bad = 0;
+    const long ntiles = ((long)n + kValRows - 1) / kValRows;
+    for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int r0 = (int)(t * kValRows), nr = min(kValRows, n - r0), r = r0 + tid;
+        __syncthreads();   // the tile before this one has been read
+        for (int i = tid; i <= nr; i += kValRows) rows_s[i] = __ldg(row + r0 + i);
+        __syncthreads();
+        int b = 0, e = 0;
+        bool ok = true;
+        if (tid < nr) {
+            b = rows_s[tid];
+            e = rows_s[tid + 1];
             if (r == 0 && b != 0) bad |= ERR_ROW0;
             if (r == n - 1 && (long long)e != nnz) bad |= ERR_ROWN;
-            if (e < b || b < 0 || (long long)e > nnz) {
-                bad |= ERR_ROWORDER;
-            } else {
-                bool diag = false;
-                int carry = 0;
-                constexpr int U = 4;   // chunks of S entries whose columns are requested together
-                for (int j00 = b; j00 < e; j00 += U * S) {
-                    int cv[U];
-#pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        const int j = j00 + u * S + lane;
-                        cv[u] = j < e ? __ldcs(col + j) : 0x7fffffff;
+            ok = !(e < b || b < 0 || (long long)e > nnz);
+            if (!ok) bad |= ERR_ROWORDER;
+            else mx = max(mx, e - b);
+        }
+        const bool all_ok = __syncthreads_and(ok);
+        const int b0 = rows_s[0];
+        const long total = all_ok ? (long)rows_s[nr] - b0 : 0;   // the rows' ranges follow one another
+        if (all_ok && total <= kValCap) {
+            for (int j = tid; j < (int)total; j += kValRows)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(cols_s + val_slot(j))),
+                    "l"(col + b0 + j) : "memory");
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (tid < nr) {
+                int prev = -1, d = -1;
+                for (int j = b - b0; j < e - b0; j++) {
+                    const int c = cols_s[val_slot(j)];
+                    if (c < 0 || c >= m) bad |= ERR_COLRANGE;
+                    if (j > b - b0 && prev >= c) bad |= ERR_COLSORT;
+                    if (c == r) d = j;
+                    if (OFFS) {
+                        const int off = c - r;
+                        mo = max(mo, off < 0 ? -off : off);
+                        cols_s[val_slot(j)] = max(-32768, min(32767, off));
                     }
-#pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        const int j0 = j00 + u * S;
-                        if (j0 >= e) break;   // uniform across the row's lanes
-                        const int j = j0 + lane;
-                        const int c = cv[u];
-                        int prev = __shfl_up_sync(mask, c, 1, S);
-                        if (lane == 0) prev = carry;
-                        if (j < e) {
-                            if (c < 0 || c >= m) bad |= ERR_COLRANGE;
-                            if (j > b && prev >= c) bad |= ERR_COLSORT;
-                            if (c == (int)r) {
-                                diag = true;
-                                if (dpos) dpos[r] = j;
-                            }
-                            const int off = c - (int)r;
-                            mo = max(mo, off < 0 ? -off : off);
-                            if (dcol) dcol[j] = (short)max(-32768, min(32767, off));
-                        }
-                        carry = __shfl_sync(mask, c, S - 1, S);
+                    prev = c;
+                }
+                if (need_diag && d < 0) bad |= ERR_NODIAG;
+                if (OFFS && dpos) dpos[r] = d < 0 ? -1 : b0 + d;
+            }
+            if (OFFS && dcol) {
+                __syncthreads();
+                for (int j = tid; j < (int)total; j += kValRows) dcol[b0 + j] = (short)cols_s[val_slot(j)];
+            }
+        } else {
+            for (int i = tid >> 5; i < nr; i += kValRows / 32) {
+                const int rb = rows_s[i], re = rows_s[i + 1], rr = r0 + i;
+                if (re < rb || rb < 0 || (long long)re > nnz) continue;   // noted above
+                int d = -1;
+                for (int j = rb + lane; j < re; j += 32) {
+                    const int c = col[j];
+                    if (c < 0 || c >= m) bad |= ERR_COLRANGE;
+                    if (j > rb && col[j - 1] >= c) bad |= ERR_COLSORT;
+                    if (c == rr) d = j;
+                    if (OFFS) {
+                        const int off = c - rr;
+                        mo = max(mo, off < 0 ? -off : off);
+                        if (dcol) dcol[j] = (short)max(-32768, min(32767, off));
                     }
                 }
-                diag = (__ballot_sync(mask, diag) & mask) != 0;
-                if (need_diag && !diag) bad |= ERR_NODIAG;
-                if (dpos && !diag && lane == 0) dpos[r] = -1;
-                mx = max(mx, e - b);
+                d = __reduce_max_sync(0xffffffffu, d);
+                if (need_diag && d < 0) bad |= ERR_NODIAG;
+                if (OFFS && dpos && lane == 0) dpos[rr] = d;
             }
         }
-        bad = __reduce_or_sync(0xffffffffu, bad);
-        if ((threadIdx.x & 31) == 0 && bad) atomicOr(err, bad);
     }
+    bad = __reduce_or_sync(0xffffffffu, bad);
     mx = __reduce_max_sync(0xffffffffu, mx);
     mo = __reduce_max_sync(0xffffffffu, mo);
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) {
+        if (bad) atomicOr(err, bad);
         if (mx > 0) atomicMax(max_row, mx);
-        if (mo > 0) atomicMax(max_off, mo);
+        if (OFFS && mo > 0) atomicMax(max_off, mo);
     }
 }
 
@@ -1526,18 +1528,21 @@ void edge_weights_dev(int n, int64_t nnz, const int* row, const int* col, const 
     BCMGX_CHECK_LAUNCH();
 }
 
-void validate_csr_dev(int n, int m, int64_t nnz, const int* row, const int* col, bool need_diag, cudaStream_t s)
+int validate_csr_dev(int n, int m, int64_t nnz, const int* row, const int* col, bool need_diag, cudaStream_t s)
 {
-    DBuf<int> err, mx;
-    err.alloc(1, s);
-    mx.alloc(1, s);
-    BCMGX_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
-    BCMGX_CUDA(cudaMemsetAsync(mx.p, 0, sizeof(int), s));
+    DBuf<int> st;   // error bits, longest row
+    st.alloc(2, s);
+    BCMGX_CUDA(cudaMemsetAsync(st.p, 0, 2 * sizeof(int), s));
+    auto k = k_validate<false>;
     note_launch();
-    k_validate<<<warp_grid(n), 256, 0, s>>>(n, m, nnz, row, col, err.p, mx.p, need_diag ? 1 : 0);
+    k<<<fit_grid(k, kValRows, ((long)n + kValRows - 1) / kValRows), kValRows, 0, s>>>(n, m, nnz, row, col, st.p, st.p + 1,
+        nullptr, nullptr, need_diag ? 1 : 0, nullptr);
     BCMGX_CHECK_LAUNCH();
-    const int e = read_err(err.p, s);
-    if (e) throw Error(BCMGX_ERR_INVALID_INPUT, "input matrix: " + err_text(e));
+    int h[2] = { 0, 0 };
+    BCMGX_CUDA(cudaMemcpyAsync(h, st.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaStreamSynchronize(s));
+    if (h[0]) throw Error(BCMGX_ERR_INVALID_INPUT, "input matrix: " + err_text(h[0]));
+    return h[1];
 }
 
 void tpos_dev(int n, int64_t nnz, const int* row, const int* col, int* tpos, cudaStream_t s)
@@ -2473,8 +2478,9 @@ void build_hierarchy(bcmgx_hierarchy* H, const bcmgx_csr* Ain)
         if (want16) A.dcol.alloc(A.nnz, s);
         const bool bcmg = P.preconditioner == BCMGX_PREC_BCMG;
         if (bcmg) A.dpos.alloc(A.n, s);
-        note_launch(); k_validate_offsets<<<gs_grid((long)A.n * 8), 256, 0, s>>>(A.n, A.m, A.nnz, A.row.p, A.col.p,
-            st.p, st.p + 1, st.p + 2, want16 ? A.dcol.p : nullptr, bcmg ? 1 : 0, bcmg ? A.dpos.p : nullptr);
+        auto k = k_validate<true>;
+        note_launch();
+        k<<<fit_grid(k, kValRows, ((long)A.n + kValRows - 1) / kValRows), kValRows, 0, s>>>(A.n, A.m, A.nnz, A.row.p, A.col.p, st.p, st.p + 1, st.p + 2, want16 ? A.dcol.p : nullptr, bcmg ? 1 : 0, bcmg ? A.dpos.p : nullptr);
         BCMGX_CHECK_LAUNCH();
         int h[3] = { 0, 0, 0 };
         BCMGX_CUDA(cudaMemcpyAsync(h, st.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -2641,7 +2647,9 @@ static void edge_weights_noalloc(int n, int64_t nnz, const int* row, const int* 
     note_launch();
     k_noalloc_reset<<<1, 1, 0, s>>>(minb, err, mx);
     note_launch();
-    k_validate<<<warp_grid(n), 256, 0, s>>>(n, n, nnz, row, col, err, mx, 1);
+    auto k = k_validate<false>;
+    k<<<fit_grid(k, kValRows, ((long)n + kValRows - 1) / kValRows), kValRows, 0, s>>>(n, n, nnz, row, col, err, mx, nullptr,
+        nullptr, 1, nullptr);
     BCMGX_CHECK_LAUNCH();
     int e = read_err(err, s);
     if (e) throw Error(BCMGX_ERR_INVALID_INPUT, "input matrix: " + err_text(e));
