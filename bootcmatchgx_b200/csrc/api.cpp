@@ -213,6 +213,19 @@ void choose_level_kernels(bcmgx_hierarchy* H)
         V.A.tpr = code < 0 ? -code : code;
         if (V.A.tpr < 1) V.A.tpr = default_tpr(V.A.n, V.A.nnz);
     }
+    if (p->preconditioner != BCMGX_PREC_BCMG) return;
+    for (int l = 0; l < L; l++) {
+        Level& V = H->lv[l];
+        const int k = l == L - 1 ? p->relaxnumber_coarse : std::max(p->prerelax_sweeps, p->postrelax_sweeps);
+        const bool f32 = p->vcycle_precision == BCMGX_VCYCLE_FP32 && l < L - 1;
+        // a level that is not tuned takes 2 threads per row where it would take 4: a cluster's chain is
+        // bound by bank conflicts of the gathers, which neighbouring rows have fewer of (20 sweeps of
+        // 3,300 rows: 34.5 us with 4, 31 with 2, 35 with 1; of 7,900 rows: 73, 57, 54)
+        const int tpr = V.A.tpr;
+        if (force.empty() && tpr == 4 && !(p->autotune && V.A.n >= kTuneMinRows)) V.A.tpr = 2;
+        build_chain(V, f32, k, H->stream);
+        if (!V.chain) V.A.tpr = tpr;
+    }
 }
 
 static bcmgx_hierarchy* setup_one(const bcmgx_csr* A, const bcmgx_params* p, int device, bool own_stream)

@@ -248,6 +248,7 @@ struct Level {
     // V-cycle work vectors
     DBuf<double> rhs, x, x2;
     DBuf<float> rhs32, x32, x232;
+    std::unique_ptr<ChainPlan> chain;   // null: one launch per sweep
 };
 
 struct SweepRecord {
@@ -490,6 +491,11 @@ constexpr int kTuneMinRows = 20000;   // rows of the smallest level that the aut
 // need64: see build_stencil
 int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s);
 void choose_level_kernels(bcmgx_hierarchy* H);
+// Sweep chains of a small level in one cluster (chain.cu): the plan (one host round trip; none when
+// the level does not fit, its longest chain of k sweeps is better as launches, or BCMGX_CHAIN=0), and k
+// sweeps from src (null: zero) into dst in the level's precision; false when they are not for a cluster.
+void build_chain(Level& V, bool f32, int k, cudaStream_t s);
+bool run_chain(const Level& V, bool f32, int k, const void* f, const void* src, void* dst, const int* skip, cudaStream_t s);
 void stage_fault_init();
 void stage_fault_check();
 int default_tpr(int n, int64_t nnz);

@@ -2199,11 +2199,6 @@ void build_patterns(DevCsr& A, cudaStream_t s)
     A.patw = W;
 }
 
-void finish_level_matrix(Level& V, bool want_f32, cudaStream_t s)
-{
-    const int n = V.A.n;
-    build_offsets(V.A, s);
-    V.M.alloc(n, s);
 // ---- stencil form ------------------------------------------------------------------------------
 // Hashes of every row's offsets (ho) and of its offsets and values (hf), 63 bits each.
 __global__ void k_st_hash(int n, const int* __restrict__ row, const int* __restrict__ col, const double* __restrict__ val,
@@ -2389,6 +2384,11 @@ void build_stencil(DevCsr& A, bool need64, cudaStream_t s)
     A.st_box = stencil_box(u, so);
 }
 
+void finish_level_matrix(Level& V, bool want_f32, cudaStream_t s)
+{
+    const int n = V.A.n;
+    build_offsets(V.A, s);
+    V.M.alloc(n, s);
     if (want_f32) V.M32.alloc(n, s);
     note_launch(); k_abs_row_sum<<<gs_grid(n), 256, 0, s>>>(n, V.A.row.p, V.A.val.p, V.M.p, want_f32 ? V.M32.p : nullptr);
     if (want_f32) {

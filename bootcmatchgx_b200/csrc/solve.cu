@@ -970,6 +970,7 @@ struct Cycle {
             copy(src, other, n);
             src = other;
         }
+        if (chain_in_cluster(l, k, f, src, dst, fcopy)) return;
         if (chain_in_block(l, k, f, src, dst, A, Bf, fcopy)) return;
         Vec fl = f;
         for (int i = 0; i < k; i++) {
@@ -980,6 +981,17 @@ struct Cycle {
                 sweep(l, fl, i == 0 ? src : out[i - 1], out[i]);
             }
         }
+    }
+
+    // A chain of a small single-vector level whose vectors all have the level's precision, as one
+    // cluster launch (chain.cu); not in the batch graph, where the clusters of many systems would
+    // wait for one another's SMs.
+    bool chain_in_cluster(int l, int k, Vec f, Vec src, Vec dst, Vec fcopy) const
+    {
+        const bool f32 = lf32(l);
+        if (rec || H->chain_in_block || lk >= 0 || fcopy.p || f.f32 != f32 || dst.f32 != f32 || (src.p && src.f32 != f32))
+            return false;
+        return run_chain(lv(l), f32, k, f.p, src.p, dst.p, skip, s);
     }
 
     // While the batch graph is captured (H->chain_in_block), a chain of k >= 2 sweeps on a small
@@ -1928,6 +1940,7 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (best != kSlicedCode) release_sliced(A);
+    if (best != kStencilCode) release_stencil(A);
     std::lock_guard<std::mutex> g(g_tune_mu);
     g_tune_cache[key] = best;
     tune_cache_store(key, best);
@@ -1940,7 +1953,6 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
 template <int S>
 __global__ void __launch_bounds__(256) k_grad_pattern(int n, const int* __restrict__ row, const int* __restrict__ col,
     const double* __restrict__ lam, const double* __restrict__ x, double* __restrict__ dA)
-    if (best != kStencilCode) release_stencil(A);
 {
     const int lane = threadIdx.x & (S - 1);
     const long stride = (long)gridDim.x * blockDim.x / S;
@@ -2113,6 +2125,7 @@ struct BatchCaptureMode {
         for (Level& V : H->lv) {
             staged.push_back((V.A.staged ? 1 : 0) | (V.A.sliced ? 2 : 0) | (V.A.stencil ? 4 : 0));
             V.A.staged = false;
+            V.A.stencil = false;
             V.A.sliced = false;
         }
     }
@@ -2122,10 +2135,10 @@ struct BatchCaptureMode {
         for (size_t l = 0; l < staged.size(); l++) {
             H->lv[l].A.staged = (staged[l] & 1) != 0;
             H->lv[l].A.sliced = (staged[l] & 2) != 0;
+            H->lv[l].A.stencil = (staged[l] & 4) != 0;
         }
     }
 };
-            V.A.stencil = false;
 
 void batch_build(bcmgx_batch* B)
 {
@@ -2135,7 +2148,6 @@ void batch_build(bcmgx_batch* B)
         ensure_solve_workspace(H);
         BatchCaptureMode mode(H);
         add_solve_to_graph(H, g);
-            H->lv[l].A.stencil = (staged[l] & 4) != 0;
     }
     BCMGX_CUDA(cudaGraphInstantiate(&B->exec, g, 0));
     BCMGX_CUDA(cudaGraphDestroy(g));

@@ -1,0 +1,74 @@
+"""Sweep chains of small levels in one thread-block cluster (chain.cu) against one launch per sweep
+(BCMGX_CHAIN=0): the same rows, order of additions and update, so cycles and solves agree bit for bit."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from test_gpu_parity import fcg
+from test_gpu_staged import matrix
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def multi_launch_cycle(monkeypatch):
+    """These tests exercise the cycle's own kernels: the persistent coarse cycle stays off."""
+    monkeypatch.setenv("BCMGX_PERSIST_NNZ", "0")
+
+
+def cycle_and_solve(bx, monkeypatch, A, chain, S=2, **kw):
+    """One cycle and one solve with S threads per row on every level."""
+    import torch
+    monkeypatch.setenv("BCMGX_CHAIN", chain)
+    monkeypatch.setenv("BCMGX_TPR", str(S))
+    n = A.shape[0]
+    h = bx.prec_setup(A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data,
+                      fcg(bx, rtol=1e-8, **kw))
+    rng = np.random.default_rng(7)
+    r = rng.uniform(-1, 1, n)
+    c0 = bx.lib().bcmgx_launch_count()
+    v = h.prec_apply(torch.from_numpy(r).cuda()).cpu().numpy()
+    launches = bx.lib().bcmgx_launch_count() - c0
+    # (one row: the start-up step is exact and leaves a zero residual, which the iteration refuses)
+    x, info = h.solve(A @ rng.uniform(-1, 1, n)) if n > 1 else (v, {"niter": 1})
+    h.free()
+    return v, x, info, launches
+
+
+# one row; a block's first rows (1 block), several blocks, the largest cluster; rows of 7 and 27 entries, random
+# columns (every block in every other's halo), a dense row, and a level too large for a cluster (it keeps its launches)
+CASES = {
+    "one_row": lambda bx: sp.identity(1, format="csr") * 3.0,
+    "lap7_tiny": lambda bx: matrix(bx, ("lap7", (5, 3, 2))),
+    "lap7": lambda bx: matrix(bx, ("lap7", (13, 11, 9))),
+    "lap27": lambda bx: matrix(bx, ("lap27", (17, 13, 11))),
+    "lap27_16": lambda bx: matrix(bx, ("lap27", (23, 21, 19))),
+    "rand": lambda bx: matrix(bx, ("rand", (5000, 0.003, 2, True))),
+    "arrow": lambda bx: matrix(bx, ("arrow", (3000, 4, 5))),
+    "diff": lambda bx: matrix(bx, ("diff", (24, 3))),
+    "lap7_large": lambda bx: matrix(bx, ("lap7", (40, 40, 40))),
+}
+
+
+@pytest.mark.parametrize("prec", ["FP64", "FP32"])
+@pytest.mark.parametrize("name,S", [(k, 2) for k in CASES] + [(k, S) for k in ("lap7", "lap27_16", "rand") for S in (1, 4, 8, 16)])
+def test_chain_bit_identical(bx, cuda, monkeypatch, name, S, prec):
+    A = CASES[name](bx)
+    A.sort_indices()
+    v0, x0, i0, l0 = cycle_and_solve(bx, monkeypatch, A, "0", S, vcycle_precision=prec)
+    v1, x1, i1, l1 = cycle_and_solve(bx, monkeypatch, A, "1", S, vcycle_precision=prec)
+    assert np.array_equal(v0, v1)
+    assert i0["niter"] == i1["niter"] and np.array_equal(x0, x1)
+    if name.startswith("lap"):
+        assert l1 < l0   # the coarsest level's chain at least is one launch
+
+
+@pytest.mark.parametrize("kw", [dict(cycle_type="W_CYCLE"), dict(cycle_type="H_CYCLE"), dict(relaxnumber_coarse=2),
+                                dict(prerelax_sweeps=1, postrelax_sweeps=2), dict(prerelax_sweeps=0, postrelax_sweeps=3),
+                                dict(use_graph=0)])
+def test_chain_cycles(bx, cuda, monkeypatch, kw):
+    """Second visits of a level (a chain from its iterate), chains of 1 to 3 sweeps, the stream driver."""
+    A = matrix(bx, ("lap7", (40, 37, 33)))
+    v0, x0, i0, _ = cycle_and_solve(bx, monkeypatch, A, "0", **kw)
+    v1, x1, i1, _ = cycle_and_solve(bx, monkeypatch, A, "1", **kw)
+    assert np.array_equal(v0, v1) and i0["niter"] == i1["niter"] and np.array_equal(x0, x1)
