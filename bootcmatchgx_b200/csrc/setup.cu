@@ -658,114 +658,140 @@ __global__ void k_logw(int n, const int* __restrict__ row, const int* __restrict
 
 // Per row: rank of every candidate (off-diagonal, W > 0) in the row's preference order,
 // (W, column) descending (find_Candidate, suitor.cu:80-147).
-// Ranks of a row of at most 32 entries held in registers (lane = entry t = b + lane, column ct
-// and weight wt; ct = -1 past the row). When the weights differ, every lane compares its entry
-// with all of the row's: the row's (weight, column) keys go to the warp's slots in shared memory
-// (`keys`, 32 per warp) and are read back as broadcasts, one 16-byte load per compared entry
-// (three shuffles per entry made shuffle throughput the bound).
-struct alignas(16) RankKey {
-    double w;
-    int c;     // column, -1 for an entry that is not a candidate
-    int pad;
-};
-__device__ __forceinline__ void rank_row32(long r, int b, int e, int ct, double wt, int* __restrict__ rank,
-    int* __restrict__ degE, RankKey* keys)
+// Ranks of rows of at most S entries (8, 16 or 32), one sub-warp of S lanes a row and one entry a lane
+// (weight w of the lane's entry, el: it is a candidate). When a row's weights differ, its lanes write
+// theirs to the warp's slots in shared memory (`keys`, 32 per warp) and count the greater ones, read back
+// as broadcasts: a load, a comparison and an addition per entry; equal weights come from one
+// match-any, and their order, by column, is the lanes'.
+template <int S>
+__device__ __forceinline__ int rank_rows(bool el, double w, int d, double* keys, unsigned* elig_out)
 {
-    const int lane = threadIdx.x & 31;
-    const int t = b + lane;
-    const bool in = t < e;
-    const bool el = in && ct != r && wt > 0.0;
-    const unsigned elig = __ballot_sync(0xffffffffu, el);
+    const int lane = threadIdx.x & 31, ls = lane & (S - 1), shift = lane & ~(S - 1);
+    const unsigned sub = S == 32 ? 0xffffffffu : ((1u << S) - 1u) << shift;
+    const unsigned eb = __ballot_sync(0xffffffffu, el) & sub;
+    const unsigned elig = eb >> shift;
+    *elig_out = elig;
+    const unsigned above = ls == 31 ? 0u : 0xffffffffu << (ls + 1);   // the row's later entries
+    const double w0 = __shfl_sync(0xffffffffu, w, eb ? __ffs(eb) - 1 : lane);
+    if (__ballot_sync(0xffffffffu, el && w != w0) == 0u) return __popc(elig & above);
+    __syncwarp();   // the warp's previous rows have been read
+    keys[lane] = el ? w : -1.0;   // candidates' weights are positive
+    __syncwarp();
     int rk = 0;
-    const double w0 = __shfl_sync(0xffffffffu, wt, elig ? __ffs(elig) - 1 : 0);
-    if (__ballot_sync(0xffffffffu, el && wt != w0) == 0u) {
-        // all candidates weigh the same: the order is by column alone (columns ascend with the
-        // lane), so the rank is the number of candidates in higher lanes
-        rk = __popc(lane == 31 ? 0u : (elig >> (lane + 1)));
+    const double* kr = keys + shift;
+    if (S == 32) {
+        for (int k = 0; k < d; k++) rk += kr[k] > w ? 1 : 0;
     } else {
-        __syncwarp();   // the warp's previous row has been read
-        keys[lane].w = wt;
-        keys[lane].c = el ? ct : -1;
-        __syncwarp();
-        const int d = e - b;
-        for (int k = 0; k < d; k++) {
-            const RankKey q = keys[k];
-            rk += (q.c >= 0 && (q.w > wt || (q.w == wt && q.c > ct))) ? 1 : 0;
-        }
+#pragma unroll
+        for (int k = 0; k < S; k++) rk += kr[k] > w ? 1 : 0;
     }
-    if (in) rank[t] = el ? rk : -1;
-    if (lane == 0) degE[r] = __popc(elig);
+    const unsigned same = __match_any_sync(0xffffffffu, (unsigned long long)__double_as_longlong(w)) & eb;
+    return rk + __popc((same >> shift) & above);
 }
 
-// k_rank for a matrix whose rows all have at most 32 entries, with every entry's weight formed
-// in registers by k_logw's expression (same operations, same rounding) instead of read from W:
-// the weights are never stored. A warp's rows are pipelined two deep: while it ranks row r, the
-// columns and transposed positions of its next row and the bounds of the row after are in
-// flight, so a row costs one memory round trip instead of three dependent ones.
-__global__ void __launch_bounds__(256, 8) k_rank_w(int n, const int* __restrict__ row, const int* __restrict__ col, const double* __restrict__ val,
-    const double* __restrict__ w, const double* __restrict__ C, const int* __restrict__ tpos, double zero_sub,
-    int* __restrict__ rank, int* __restrict__ degE, const double* __restrict__ zero_sub_dev)
+// The ranks of a matrix whose rows all have at most S entries. FUSED: every entry's weight is formed in
+// registers by k_logw's expression (same operations, same rounding) instead of read from W, so the
+// weights are never stored, and where the row allows it the logarithm is left out: the order of the
+// logarithms is that of their arguments unless two of them are within rounding of each other
+// (kRankNear, far above the logarithm's error at any argument), and a logarithm is positive exactly when
+// its argument exceeds 1. A warp that finds two neighbours in its rows' order that close, and not equal,
+// ranks its rows again by the logarithms. A warp's rows are pipelined two deep: while it ranks its
+// rows, the columns and transposed positions (FUSED, else the weights) of the next rows and the bounds of
+// those after are in flight. Bound by instruction issue, hence the sub-warps: with a warp a row a 7-point
+// row left 25 of 32 lanes idle. Set-up of 7-point 256^3 diffusion: 15.1 -> 7.2 ms over its 10 sweeps, of
+// 27-point 160^3 3.9 -> 2.6 ms (full warps; the logarithm and the two-word comparisons gone).
+constexpr double kRankNear = 1e-12;
+template <int S, bool FUSED>
+__global__ void __launch_bounds__(256, 6) k_rank_rows(int n, const int* __restrict__ row, const int* __restrict__ col,
+    const double* __restrict__ val, const double* __restrict__ w, const double* __restrict__ C, const int* __restrict__ tpos,
+    double zero_sub, const double* __restrict__ W, int* __restrict__ rank, int* __restrict__ degE,
+    const double* __restrict__ zero_sub_dev)
 {
-    if (zero_sub_dev) zero_sub = *zero_sub_dev;
-    const int lane = threadIdx.x & 31;
-    __shared__ RankKey keys[8][32];   // 256-thread blocks
-    RankKey* wkeys = keys[(threadIdx.x >> 5) & 7];
-    const long step = (long)gridDim.x * blockDim.x / 32;
-    long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32;   // uniform across the warp
-    if (r >= n) return;
-    int b = __ldg(row + r), e = __ldg(row + r + 1);
-    int ct = b + lane < e ? __ldg(col + b + lane) : -1;
-    int tp = b + lane < e ? __ldg(tpos + b + lane) : -1;
-    long r1 = r + step;
-    int b1 = 0, e1 = 0;
-    if (r1 < n) {
-        b1 = __ldg(row + r1);
-        e1 = __ldg(row + r1 + 1);
-    }
-    while (true) {
-        const long r2 = r1 + step;
-        int b2 = 0, e2 = 0;
-        if (r2 < n) {
-            b2 = __ldg(row + r2);
-            e2 = __ldg(row + r2 + 1);
+    if (FUSED && zero_sub_dev) zero_sub = *zero_sub_dev;
+    constexpr int RW = 32 / S;   // rows of a warp
+    const int lane = threadIdx.x & 31, ls = lane & (S - 1), shift = lane & ~(S - 1);
+    __shared__ double keys[8][32];   // 256-thread blocks
+    double* wkeys = keys[(threadIdx.x >> 5) & 7];
+    const long step = (long)gridDim.x * blockDim.x / 32 * RW;
+    const long w0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * RW;   // the warp's first row
+    if (w0 >= n) return;
+    long r = w0 + lane / S;
+    auto bounds = [&](long q, int& b, int& e) {
+        b = e = 0;
+        if (q < n) {
+            b = __ldg(row + q);
+            e = __ldg(row + q + 1);
         }
-        int ct1 = -1, tp1 = -1;
-        if (b1 + lane < e1) {
-            ct1 = __ldg(col + b1 + lane);
-            tp1 = __ldg(tpos + b1 + lane);
+    };
+    int b, e, b1, e1, ct, tp = -1;
+    double wv = 0.0;
+    auto fetch = [&](int bb, int ee, int& c, int& t, double& v) {
+        const int j = bb + ls;
+        c = t = -1;
+        v = 0.0;
+        if (j < ee) {
+            c = __ldg(col + j);
+            if (FUSED) t = __ldg(tpos + j);
+            else v = __ldg(W + j);
         }
-        const int t = b + lane;
-        double wt = 0.0;
-        if (ct >= 0 && ct != (int)r) {
+    };
+    bounds(r, b, e);
+    fetch(b, e, ct, tp, wv);
+    bounds(r + step, b1, e1);
+    for (long base = w0; base < n; base += step, r += step) {
+        int b2, e2, ct1, tp1;
+        double wv1;
+        bounds(r + 2 * step, b2, e2);
+        fetch(b1, e1, ct1, tp1, wv1);
+        const int t = b + ls;
+        const bool off = ct >= 0 && ct != (int)r;
+        double x = wv;
+        if (FUSED && off) {
             const int src = (ct < (int)r && tp >= 0) ? tp : t;
             const double sa = fabs(ahat(__ldg(val + src), __ldg(C + r), __ldg(C + ct), __ldg(w + r), __ldg(w + ct)));
-            wt = log(sa != 0.0 ? sa : zero_sub);
+            x = sa != 0.0 ? sa : zero_sub;
         }
-        rank_row32(r, b, e, ct, wt, rank, degE, wkeys);
-        if (r1 >= n) break;
-        r = r1;
+        const bool el = off && (FUSED ? x > 1.0 : x > 0.0);
+        unsigned elig;
+        int rk = rank_rows<S>(el, x, e - b, wkeys, &elig);
+        if (FUSED) {
+            __syncwarp();
+            if (el) wkeys[shift + rk] = x;   // in order
+            __syncwarp();
+            const double next = el && rk + 1 < __popc(elig) ? wkeys[shift + rk + 1] : x;
+            const bool near = el && next != x && x - next <= kRankNear * x;
+            if (__any_sync(0xffffffffu, near)) rk = rank_rows<S>(el, el ? log(x) : 0.0, e - b, wkeys, &elig);
+        }
+        if (t < e) rank[t] = el ? rk : -1;
+        if (ls == 0 && r < n) degE[r] = __popc(elig);
         b = b1;
         e = e1;
         ct = ct1;
         tp = tp1;
-        r1 = r2;
+        wv = wv1;
         b1 = b2;
         e1 = e2;
     }
 }
 
+// The ranks where some row has more than 32 entries: a warp a row, every lane counting over the row.
 __global__ void k_rank(int n, const int* __restrict__ row, const int* __restrict__ col, const double* __restrict__ W,
     int* __restrict__ rank, int* __restrict__ degE)
 {
     const int lane = threadIdx.x & 31;
-    __shared__ RankKey keys[8][32];   // 256-thread blocks
-    RankKey* wkeys = keys[(threadIdx.x >> 5) & 7];
+    __shared__ double keys[8][32];   // 256-thread blocks
+    double* wkeys = keys[(threadIdx.x >> 5) & 7];
     for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32; r < n; r += (long)gridDim.x * blockDim.x / 32) {
         const int b = row[r], e = row[r + 1];
         if (e - b <= 32) {
             const int t = b + lane;
             const bool in = t < e;
-            rank_row32(r, b, e, in ? col[t] : -1, in ? W[t] : 0.0, rank, degE, wkeys);
+            const double wt = in ? W[t] : 0.0;
+            const bool el = in && col[t] != (int)r && wt > 0.0;
+            unsigned elig;
+            const int rk = rank_rows<32>(el, wt, e - b, wkeys, &elig);
+            if (in) rank[t] = el ? rk : -1;
+            if (lane == 0) degE[r] = __popc(elig);
             continue;
         }
         int cnt = 0;
@@ -1577,10 +1603,21 @@ void suitor_dev(int n, int64_t nnz, const int* row, const int* col, const double
         offer.alloc(n, s);
         BCMGX_CUDA(cudaMemsetAsync(offer.p, 0, sizeof(unsigned) * n, s));
     }
-    if (fw) {
+    auto ranks = [&](auto kern, int S) {
+        const FusedWeights none;
+        const FusedWeights& f = fw ? *fw : none;
         note_launch();
-        k_rank_w<<<warp_grid(n), 256, 0, s>>>(n, row, col, fw->val, fw->w, fw->C, tpos, fw->zero_sub, rank.p, degE.p,
-            fw->zero_sub_dev);
+        kern<<<gs_grid((long)n * S), 256, 0, s>>>(n, row, col, f.val, f.w, f.C, tpos, f.zero_sub, W, rank.p, degE.p,
+            f.zero_sub_dev);
+    };
+    if (fw) {
+        if (max_row <= 8) ranks(k_rank_rows<8, true>, 8);
+        else if (max_row <= 16) ranks(k_rank_rows<16, true>, 16);
+        else ranks(k_rank_rows<32, true>, 32);
+    } else if (max_row <= 32) {
+        if (max_row <= 8) ranks(k_rank_rows<8, false>, 8);
+        else if (max_row <= 16) ranks(k_rank_rows<16, false>, 16);
+        else ranks(k_rank_rows<32, false>, 32);
     } else {
         note_launch(); k_rank<<<warp_grid(n), 256, 0, s>>>(n, row, col, W, rank.p, degE.p);
     }
@@ -2098,13 +2135,19 @@ __global__ void k_pat_hash(int n, const int* __restrict__ row, const short* __re
 }
 
 // rep[id] = some row of form id; len[id] its length. The claim is tried only while the form has
-// none (a plain load first): millions of rows share a few forms, and atomics on one word serialise.
+// none and the block has not seen it before: millions of rows share a few forms, and loads and
+// atomics on one word serialise (27-point 160^3: 209 us with a load by every row).
 __global__ void k_pat_rep(int n, const int* __restrict__ row, const unsigned char* __restrict__ pid, int* rep,
     int* len)
 {
+    __shared__ unsigned char seen[256];   // forms that this block knows to be claimed
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) seen[i] = 0;
+    __syncthreads();
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
         const int id = pid[r];
+        if (((volatile unsigned char*)seen)[id]) continue;
         if (ld_cg(rep + id) == -1 && atomicCAS(rep + id, -1, (int)r) == -1) len[id] = row[r + 1] - row[r];
+        ((volatile unsigned char*)seen)[id] = 1;
     }
 }
 
