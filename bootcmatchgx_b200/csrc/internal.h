@@ -327,6 +327,7 @@ struct bcmgx_hierarchy {
     bool chain_in_block = false;        // small levels' sweep chains as one-block kernels (batch graphs)
     // captured solve (CUDA graph) and its own b / x buffers
     cudaGraphExec_t iter_graph = nullptr;
+    int solves = 0;   // solves so far (fcg_solve)
     bcmgx::DBuf<double> gb, gx;
     long long graph_startup_kernels = 0, graph_body_kernels = 0;
     bcmgx::CycleBufs cyc;                 // single-vector cycle buffers (views of lv[l] and res)
