@@ -323,11 +323,12 @@ def vcycle_bytes(inf, pre, post, coarse):
     prolongation x += p x_c[agg]; the coarsest level runs `coarse` FP64 sweeps (the first from
     zero). Matrix entries
     count index_bytes + value bytes (1 where the level streams 1-byte value codes, else 4; 8 for the
-    coarsest level's FP64 values; index_bytes 0, pattern-indexed rows, streams 1 byte per row instead),
+    coarsest level's FP64 values; index_bytes 0, pattern-indexed rows, streams 1 byte per row instead; -1, the
+    stencil form, also takes the values from a table where the level has value codes),
     vectors 4 bytes (8 on the coarsest level); level 0 also reads the FP64 residual and writes the FP64
     output."""
-    n, z, ib = inf["n"], inf["nnz"], inf["index_bytes"]
-    vb = [1 if c else 4 for c in inf["value_codes"]]
+    n, z, ib = inf["n"], inf["nnz"], [max(b, 0) for b in inf["index_bytes"]]
+    vb = [(0 if b < 0 else 1) if c else 4 for b, c in zip(inf["index_bytes"], inf["value_codes"])]
     total = 0
     for l in range(len(n) - 1):
         nl, zl, nc = n[l], z[l], n[l + 1]
@@ -451,8 +452,12 @@ def run_ours(a, wl, rank, world, local_rank):
     # row naming its offsets; 1-byte value codes where the level has them, else the 4- or 8-byte
     # values; bcmgx_spmv on raw CSR arrays always streams int32 + FP64
     ib32, ib64 = inf32["index_bytes"][0], inf64["index_bytes"][0]
-    vb32 = 1 if inf32["value_codes"][0] else 4
-    vb64 = 1 if inf64["value_codes"][0] else 8
+    # (the stencil form, index bytes -1: one byte per row, which also names the values of a level with
+    # value codes)
+    sten32, sten64 = ib32 < 0, ib64 < 0
+    ib32, ib64 = max(ib32, 0), max(ib64, 0)
+    vb32 = (0 if sten32 else 1) if inf32["value_codes"][0] else 4
+    vb64 = (0 if sten64 else 1) if inf64["value_codes"][0] else 8
     rb32, rb64 = (n if ib32 == 0 else 0), (n if ib64 == 0 else 0)
     bytes_spmv = 12 * nnz + 4 * (n + 1) + 16 * n
     bytes_jac32 = (ib32 + vb32) * nnz + rb32 + 4 * (n + 1) + 16 * n
@@ -497,9 +502,9 @@ def run_ours(a, wl, rank, world, local_rank):
     setup64 = float(np.mean([i[1]["setup_ms"] for i in infos64]))
     solve64 = float(np.mean([i[0]["solve_ms"] for i in infos64]))
     nrm = np.linalg.norm
-    tpr0 = inf32["tpr"][0]   # level 0's kernel code: threads per row, negative staged, 64 sliced
-    form0 = "sliced" if tpr0 == 64 else "staged" if tpr0 < 0 else "plain"
-    kname0 = {"sliced": "k_rowop_sliced<", "staged": f"k_rowop_staged<{-tpr0},", "plain": f"k_rowop<{tpr0},"}[form0]
+    tpr0 = inf32["tpr"][0]   # level 0's kernel code: threads per row, negative staged, 64 sliced or stencil (index bytes -1)
+    form0 = "stencil" if sten32 else "sliced" if tpr0 == 64 else "staged" if tpr0 < 0 else "plain"
+    kname0 = {"stencil": "k_rowop_box27 / k_rowop_stencil<", "sliced": "k_rowop_sliced<", "staged": f"k_rowop_staged<{-tpr0},", "plain": f"k_rowop<{tpr0},"}[form0]
     line = {
         "metric": METRIC, "value": ms32 / 1e3, "unit": "s", "n_gpus": world, "steps": a.steps,
         "warmup": a.warmup, "ms_per_step": ms32, "higher_is_better": False, "scaling": "weak",
@@ -541,8 +546,9 @@ def run_ours(a, wl, rank, world, local_rank):
         "roofline": {"kernel": (("k_rowop_slpat<OP_JACOBI,float>" if (form0 == "sliced" and ib32 == 0) else
                                  kname0 + ("OP_JACOBI,Coded<float>>" if vb32 == 1 else "OP_JACOBI,float>"))
                                 + " (FP32 l1-Jacobi sweep, level 0)"),
-                     "format": ("pattern-indexed rows (1 byte per row)" if ib32 == 0 else f"int{8 * ib32} columns")
-                               + ", " + ("1-byte value codes" if vb32 == 1 else "FP32 values"),
+                     "format": ("stencil form (1 byte per row)" if sten32 else
+                                "pattern-indexed rows (1 byte per row)" if ib32 == 0 else f"int{8 * ib32} columns")
+                               + ", " + {0: "values from a table", 1: "1-byte value codes"}.get(vb32, "FP32 values"),
                      "bound": "hbm", "achieved": gbs_jac32, "peak": peak, "unit": "GB/s",
                      "frac": gbs_jac32 / peak, "peak_kind": f"{peak_kind} hbm_gbs (copy)",
                      "bytes_per_launch": bytes_jac32,

@@ -125,10 +125,12 @@ typedef struct bcmgx_hierarchy_info {
     double setup_ms;         /* device time of the set-up (CUDA events) */
     int tpr[BCMGX_MAX_LEVELS];   /* threads per row the solve kernels use on each level; negative: the
                                     staged kernel (matrix entries through shared memory) with -tpr;
-                                    64: the sliced kernel (32-row slices, one thread per row) */
+                                    64: the sliced or stencil kernels (one thread per row) */
     int index_bytes[BCMGX_MAX_LEVELS]; /* column index bytes the solve kernels stream per entry
                                           (2: int16 offsets from the diagonal, 4: int32; 0: pattern-
-                                          indexed rows, one byte per row naming the row's offsets) */
+                                          indexed rows, one byte per row naming the row's offsets;
+                                          -1: the stencil form, where that byte also names the row's
+                                          values or they are stored by offset) */
     int value_codes[BCMGX_MAX_LEVELS]; /* distinct values of a level whose solve kernels stream
                                           one-byte value codes (value-indexed CSR), else 0 */
 } bcmgx_hierarchy_info;
