@@ -13,6 +13,7 @@
 // gathers go through L1 / L2, where neighbouring rows reuse them.
 #pragma once
 
+#include "internal.h"
 #include "common.cuh"
 
 namespace bcmgx {
@@ -294,6 +295,160 @@ __global__ void __launch_bounds__(kBlkRowopThreads, blk_min_blocks<VT, W>()) k_b
         });
 }
 
+// ---- 27-point boxes ----
+// The block products of a level in the stencil form whose offsets are a box's (stencil.cuh,
+// k_rowop_box27: pl[a] + (b - 1) s + (c - 1) for entry 9 a + 3 b + c) with its values in the forms' table.
+struct BoxArgs {
+    int s, pl0, pl2, nform;
+    const unsigned char* form;
+    const unsigned* mask;
+};
+constexpr int kBlkBoxP = 4;   // rows of a slot
+
+// As blk_rows, but a slot takes P rows s apart: they share the block rows of X that they gather (a plane's
+// P + 2 lines of three), so a row costs 9 (P + 2) / P vector loads instead of 27, and no entry is
+// staged. The entries of a row are added in CSR order; a block row of X is loaded when one of the P rows
+// has its column, and added to the rows that have it. Dynamic shared memory: 36 values a form. Bound by the
+// latency of the gathers at 32 columns (their block is larger than L2): FP32 sweeps of 27-point 100^3 take
+// 177 us instead of 217, with 8 columns 56 instead of 180, with 2 23 instead of 180.
+template <int W, int P, typename VT, typename XT, typename Epi>
+__device__ __forceinline__ void blk_box_rows(int n, int lpe_log2, int ld, int K, const BoxArgs& box,
+    const VT* __restrict__ vals, const XT* __restrict__ X, Epi&& epi)
+{
+    using AT = typename Acc<VT>::type;
+    constexpr unsigned kFull = (1u << 27) - 1u;
+    constexpr int TW = 36;   // table row: three planes of 9 values and 3 of padding
+    extern __shared__ __align__(128) unsigned char blk_box_smem[];
+    __shared__ unsigned mask_s[256];
+    VT* tab_s = (VT*)blk_box_smem;
+    for (int i = threadIdx.x; i < box.nform; i += blockDim.x) mask_s[i] = __ldg(box.mask + i);
+    for (int i = threadIdx.x; i < box.nform * TW; i += blockDim.x) {
+        const int id = i / TW, w = i % TW;
+        tab_s[i] = w % 12 < 9 ? __ldg(vals + id * 28 + (w / 12) * 9 + w % 12) : VT(0);
+    }
+    __syncthreads();
+    const int s = box.s;
+    const int lane = threadIdx.x & 31;
+    const int c0 = (lane & ((1 << lpe_log2) - 1)) * W;
+    const bool active = c0 < K;
+    const long items = ((long)n + (long)P * s - 1) / ((long)P * s) * s;
+    const long stride = (long)gridDim.x * (blockDim.x >> lpe_log2);
+    const int dq = (int)(stride / s), dt = (int)(stride % s);
+    const long warp0 = ((long)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> lpe_log2;   // the warp's first slot
+    const long i0 = warp0 + (lane >> lpe_log2);
+    int q = (int)(i0 / s), t = (int)(i0 % s);
+    for (long i = warp0; i < items; i += stride) {
+        const long base = (long)q * P * s + t;   // rows of slots past the last group are all >= n
+        int id[P];
+        unsigned m[P];
+        bool one = true;
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const long r = base + (long)p * s;
+            id[p] = r < n ? (int)__ldg(box.form + r) : -1;
+            m[p] = id[p] >= 0 ? mask_s[id[p]] : 0u;
+            one = one && id[p] == id[0];
+        }
+        const int id0 = __shfl_sync(0xffffffffu, id[0], 0);   // by every lane, whatever its rows
+        const bool inner = __all_sync(0xffffffffu, one && m[0] == kFull && id[0] == id0);
+        AT acc[P][W];
+#pragma unroll
+        for (int p = 0; p < P; p++)
+#pragma unroll
+            for (int w = 0; w < W; w++) acc[p][w] = 0;
+        if (inner) {
+            if (active) {
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    const XT* xl = X + (base + (a == 0 ? box.pl0 : a == 1 ? 0 : box.pl2) - s) * ld + c0;
+                    VT cv[9];
+#pragma unroll
+                    for (int k = 0; k < 9; k++) cv[k] = tab_s[id[0] * TW + 12 * a + k];
+#pragma unroll
+                    for (int l = 0; l < P + 2; l++) {
+                        XT x[3][W];
+#pragma unroll
+                        for (int c = 0; c < 3; c++) ldv<W>(xl + ((long)l * s + c - 1) * ld, x[c]);
+#pragma unroll
+                        for (int p = 0; p < P; p++)
+                            if (l - p >= 0 && l - p < 3)
+#pragma unroll
+                                for (int c = 0; c < 3; c++)
+#pragma unroll
+                                    for (int w = 0; w < W; w++) acc[p][w] += (AT)cv[3 * (l - p) + c] * (AT)x[c][w];
+                    }
+                }
+            }
+        } else if (active) {
+#pragma unroll 1
+            for (int a = 0; a < 3; a++) {
+                const XT* xl = X + (base + (a == 0 ? box.pl0 : a == 1 ? 0 : box.pl2) - s) * ld + c0;
+#pragma unroll
+                for (int l = 0; l < P + 2; l++) {
+                    XT x[3][W];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        bool need = false;
+#pragma unroll
+                        for (int p = 0; p < P; p++)
+                            if (l - p >= 0 && l - p < 3) need = need || ((m[p] >> (9 * a + 3 * (l - p) + c)) & 1u);
+#pragma unroll
+                        for (int w = 0; w < W; w++) x[c][w] = XT(0);
+                        if (need) ldv<W>(xl + ((long)l * s + c - 1) * ld, x[c]);
+                    }
+#pragma unroll
+                    for (int p = 0; p < P; p++)
+                        if (l - p >= 0 && l - p < 3)
+#pragma unroll
+                            for (int c = 0; c < 3; c++)
+                                if ((m[p] >> (9 * a + 3 * (l - p) + c)) & 1u) {
+                                    const AT v = (AT)tab_s[id[p] * TW + 12 * a + 3 * (l - p) + c];
+#pragma unroll
+                                    for (int w = 0; w < W; w++) acc[p][w] += v * (AT)x[c][w];
+                                }
+                }
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const long r = base + (long)p * s;
+            if (r < n && active) epi(r, r * ld + c0, acc[p]);
+        }
+        q += dq;
+        t += dt;
+        if (t >= s) {
+            t -= s;
+            q++;
+        }
+    }
+}
+
+// the row operations of k_blk_rowop on a 27-point box
+template <int OP, int W, typename VT, typename XT, typename FT, typename MT, typename YT>
+__global__ void __launch_bounds__(kBlkRowopThreads, 2) k_blk_box(int n, int lpe_log2, int ld, int K, BoxArgs box,
+    const VT* __restrict__ vals, const XT* __restrict__ X, const FT* __restrict__ F, const MT* __restrict__ M,
+    YT* __restrict__ Y, const int* __restrict__ skip)
+{
+    if (skip && *skip) return;
+    using AT = typename Acc<VT>::type;
+    blk_box_rows<W, kBlkBoxP>(n, lpe_log2, ld, K, box, vals, X, [&](long r, long o, const AT (&s)[W]) {
+        YT y[W];
+        FT f[W];
+        ldw<W>(F + o, f);
+        if (OP == 1) {
+#pragma unroll
+            for (int w = 0; w < W; w++) y[w] = (YT)((AT)f[w] - s[w]);
+        } else {
+            XT x[W];
+            ldw<W>(X + o, x);
+            const AT m = (AT)M[r];
+#pragma unroll
+            for (int w = 0; w < W; w++) y[w] = (YT)(((-s[w] + (AT)f[w]) / m) + (AT)x[w]);
+        }
+        stv<W>(Y + o, y);
+    });
+}
+
 // sweep from a zero iterate: U = F / M, optionally keeping a converted copy of F
 template <typename FT, typename MT, typename YT, typename CT>
 __global__ void k_blk_first_sweep(int n, int lk, const FT* __restrict__ F, const MT* __restrict__ M, YT* __restrict__ U,
@@ -336,6 +491,22 @@ __global__ void k_blk_prolong(int n, int lk, const int* __restrict__ agg, const 
         const long r = i >> lk;
         Y[i] = (YT)((AT)p[r] * (AT)XC[((long)agg[r] << lk) + (i & mask)] + (AT)X[i]);
     }
+}
+
+// A box level's arguments, the items of its slots (kBlkBoxP rows each) and the table's bytes.
+struct BoxLevel {
+    BoxArgs box;
+    long items;
+    size_t smem;
+};
+inline BoxLevel box_level(const DevCsr& A, size_t value_bytes)
+{
+    BoxLevel b;
+    b.box = BoxArgs { A.st_box, A.st_offs.o[4], A.st_offs.o[22], A.st_nform, A.st_form.p, A.st_mask.p };
+    const long ps = (long)kBlkBoxP * A.st_box;
+    b.items = ((long)A.n + ps - 1) / ps * A.st_box;
+    b.smem = (size_t)A.st_nform * 36 * value_bytes;
+    return b;
 }
 
 }  // namespace bcmgx

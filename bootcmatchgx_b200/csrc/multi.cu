@@ -66,11 +66,22 @@ __device__ __forceinline__ bool blk_colsum(const double (&v)[NV][W], int lpe, do
     __syncthreads();
     if (!last) return false;
     __threadfence();
+    // the blocks' sums: every warp adds each nw-th block, then warp 0 the warps', in a fixed order (by one
+    // warp alone, a chain of loads over 600 to 900 blocks, it took 80 us a sum after 390 us of update)
+    const int nw = blockDim.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        double t = 0.0;
+#pragma unroll 8
+        for (int b = wid; b < (int)gridDim.x; b += nw) t += __ldcg(partials + ((size_t)b * NV + q) * 32 + lane);
+        sh[q][wid][lane][0] = t;
+    }
+    __syncthreads();
     if (wid == 0) {
 #pragma unroll
         for (int q = 0; q < NV; q++) {
             double t = 0.0;
-            for (int b = 0; b < (int)gridDim.x; b++) t += __ldcg(partials + ((size_t)b * NV + q) * 32 + lane);
+            for (int wi = 0; wi < nw; wi++) t += sh[q][wi][lane][0];
             out[q] = t;
         }
         if (lane == 0) *ticket = 0;
@@ -125,34 +136,13 @@ __global__ void __launch_bounds__(kBlkThreads, 4) k_blk_resid0(int n, int lpe_lo
     }
 }
 
-// PW = A PV with the per-column dots alpha = r.pv, beta = pw.pv (and gamma = oq.pv in the loop),
-// then the scalar recurrence of each running column (FCG.cu:59-86, 121-136).
+// The step's sums over all blocks and its scalar recurrence, per column (k_fcg_dots).
 template <int MODE, int W>
-__global__ void __launch_bounds__(kBlkThreads, 4) k_blk_spmv_dots(int n, int lpe_log2, int kp, const int* __restrict__ row,
-    const int* __restrict__ col, const double* __restrict__ val, const double* __restrict__ PV, double* __restrict__ PW,
-    const double* __restrict__ R, const double* __restrict__ OQ, BlockState* st, double* partials, int stage_ok,
-    const int* __restrict__ skip)
+__device__ __forceinline__ void blk_dots_scalars(const double (&acc)[3][W], int lpe, int kp, BlockState* st, double* partials)
 {
-    if (skip && *skip) return;
-    __shared__ BlkEnt<double> stage[kBlkThreads / 32][BlkStage<double>::cap];
     const int lane = threadIdx.x & 31;
-    double acc[3][W] = {};
-    blk_rows<W>(n, lpe_log2, kp, kp, row, col, val, PV, stage_ok, stage[threadIdx.x >> 5],
-        [&](long, long o, const double (&s)[W]) {
-            double vi[W], ri[W], qi[W];
-            stv<W>(PW + o, s);
-            ldw<W>(PV + o, vi);
-            ldw<W>(R + o, ri);
-            if (MODE == 1) ldw<W>(OQ + o, qi);
-#pragma unroll
-            for (int w = 0; w < W; w++) {
-                acc[0][w] += ri[w] * vi[w];
-                acc[1][w] += s[w] * vi[w];
-                if (MODE == 1) acc[2][w] += qi[w] * vi[w];
-            }
-        });
     double out[3];
-    if (blk_colsum<3, W>(acc, 1 << lpe_log2, partials, &st->ticket[1], out) && threadIdx.x < kp && !st->done[lane]) {
+    if (blk_colsum<3, W>(acc, lpe, partials, &st->ticket[1], out) && threadIdx.x < kp && !st->done[lane]) {
         const int k = lane;
         st->alpha[k] = out[0];
         st->beta[k] = out[1];
@@ -169,6 +159,60 @@ __global__ void __launch_bounds__(kBlkThreads, 4) k_blk_spmv_dots(int n, int lpe
         }
         if (!(st->delta[k] > 0.0) || !isfinite(st->theta[k])) st->bad[k] = 1;
     }
+}
+
+// PW = A PV with the per-column dots alpha = r.pv, beta = pw.pv (and gamma = oq.pv in the loop),
+// then the scalar recurrence of each running column (FCG.cu:59-86, 121-136).
+template <int MODE, int W>
+__global__ void __launch_bounds__(kBlkThreads, 4) k_blk_spmv_dots(int n, int lpe_log2, int kp, const int* __restrict__ row,
+    const int* __restrict__ col, const double* __restrict__ val, const double* __restrict__ PV, double* __restrict__ PW,
+    const double* __restrict__ R, const double* __restrict__ OQ, BlockState* st, double* partials, int stage_ok,
+    const int* __restrict__ skip)
+{
+    if (skip && *skip) return;
+    __shared__ BlkEnt<double> stage[kBlkThreads / 32][BlkStage<double>::cap];
+    double acc[3][W] = {};
+    blk_rows<W>(n, lpe_log2, kp, kp, row, col, val, PV, stage_ok, stage[threadIdx.x >> 5],
+        [&](long, long o, const double (&s)[W]) {
+            double vi[W], ri[W], qi[W];
+            stv<W>(PW + o, s);
+            ldw<W>(PV + o, vi);
+            ldw<W>(R + o, ri);
+            if (MODE == 1) ldw<W>(OQ + o, qi);
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                acc[0][w] += ri[w] * vi[w];
+                acc[1][w] += s[w] * vi[w];
+                if (MODE == 1) acc[2][w] += qi[w] * vi[w];
+            }
+        });
+    blk_dots_scalars<MODE, W>(acc, 1 << lpe_log2, kp, st, partials);
+}
+
+// The same on a 27-point box (blk_box_rows): the product's gathers are what bounds it, and four rows share
+// them. 27-point 100^3: 508 -> 349 us with 32 columns, 343 -> 127 with 8, 308 -> 72 with 2 (the column sums'
+// last stage by all warps included).
+template <int MODE, int W>
+__global__ void __launch_bounds__(kBlkThreads, 2) k_blk_box_dots(int n, int lpe_log2, int kp, BoxArgs box,
+    const double* __restrict__ tab, const double* __restrict__ PV, double* __restrict__ PW, const double* __restrict__ R,
+    const double* __restrict__ OQ, BlockState* st, double* partials, const int* __restrict__ skip)
+{
+    if (skip && *skip) return;
+    double acc[3][W] = {};
+    blk_box_rows<W, kBlkBoxP>(n, lpe_log2, kp, kp, box, tab, PV, [&](long, long o, const double (&s)[W]) {
+        double vi[W], ri[W], qi[W];
+        stv<W>(PW + o, s);
+        ldw<W>(PV + o, vi);
+        ldw<W>(R + o, ri);
+        if (MODE == 1) ldw<W>(OQ + o, qi);
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+            acc[0][w] += ri[w] * vi[w];
+            acc[1][w] += s[w] * vi[w];
+            if (MODE == 1) acc[2][w] += qi[w] * vi[w];
+        }
+    });
+    blk_dots_scalars<MODE, W>(acc, 1 << lpe_log2, kp, st, partials);
 }
 
 // Start-up update of each running column (FCG.cu:88-100): X += theta V, R -= theta W, D = V,
@@ -369,6 +413,22 @@ void launch_dots(const DevCsr& A, const MultiWork& wk, const double* pv, double*
 {
     const BlkShape sh = fcg_shape(wk);
     const int kp = 1 << wk.lk;
+    if (A.stencil && A.st_box > 0 && A.st_tab64.p) {
+        auto box = [&](auto kern) {
+            const BoxLevel bl = box_level(A, sizeof(double));
+            ensure_smem_limit((const void*)kern, bl.smem);
+            const long need = ceil_div(bl.items, kBlkThreads >> sh.lpe_log2);
+            const int grid = (int)std::min<long>(std::max<long>(need, 1),
+                (long)num_sms() * std::min(blocks_per_sm((const void*)kern, kBlkThreads, bl.smem), kBlkBlocksPerSM));
+            note_launch();
+            kern<<<grid, kBlkThreads, bl.smem, s>>>(A.n, sh.lpe_log2, kp, bl.box, (const double*)A.st_tab64.p, pv, pw, wk.R.p,
+                oq, wk.st.p, wk.part.p, skip);
+        };
+        if (sh.W == 2) box(k_blk_box_dots<MODE, 2>);
+        else box(k_blk_box_dots<MODE, 1>);
+        BCMGX_CHECK_LAUNCH();
+        return;
+    }
     auto go = [&](auto kern) {
         note_launch();
         kern<<<rows_grid(kern, A.n, sh), kBlkThreads, 0, s>>>(A.n, sh.lpe_log2, kp, A.row.p, A.col.p, A.val.p, pv, pw,

@@ -661,6 +661,60 @@ static void launch_blk_rowop(int n, int m, int ld, int K, const int* row, const 
     BCMGX_CHECK_LAUNCH();
 }
 
+constexpr long kBlkBoxMin = 1 << 20;   // block entries from which the box kernel runs
+
+// A residual or a sweep on blocks of K = 2^lk columns of a level in the stencil form of a 27-point box
+// (blk_box_rows); false for any other level, vectors that are not aligned for the block's vector loads,
+// and blocks of fewer rows than give every SM work.
+template <int OP, typename VT, typename XT, typename FT, typename MT, typename YT>
+static bool launch_blk_box(const DevCsr& A, int K, const VT* val, const XT* x, const FT* f, const MT* M, YT* y,
+    const int* skip, cudaStream_t s)
+{
+    if constexpr (OP != OP_AXPBY) {
+        const VT *own, *tab;
+        if constexpr (std::is_same<VT, float>::value) {
+            own = A.val32.p;
+            tab = A.st_tab32.p;
+        } else {
+            own = A.val.p;
+            tab = A.st_tab64.p;
+        }
+        if (!A.stencil || A.st_box <= 0 || !tab || val != own || (long)A.n * K < kBlkBoxMin) return false;
+        const BlkShape sh = blk_shape(K, (int)sizeof(XT));
+        if (sh.W > 1 && (!aligned_for(x, sh.W, sizeof(XT)) || !aligned_for(y, sh.W, sizeof(YT)) || !aligned_for(f, sh.W, sizeof(FT))))
+            return false;
+        const BoxLevel bl = box_level(A, sizeof(VT));
+        auto go = [&](auto kern) {
+            ensure_smem_limit((const void*)kern, bl.smem);
+            const long need = ceil_div(bl.items, kBlkRowopThreads >> sh.lpe_log2);
+            const int grid = (int)std::max<long>(1, std::min<long>(need,
+                (long)num_sms() * blocks_per_sm((const void*)kern, kBlkRowopThreads, bl.smem)));
+            note_launch();
+            kern<<<grid, kBlkRowopThreads, bl.smem, s>>>(A.n, sh.lpe_log2, K, K, bl.box, tab, x, f, M, y, skip);
+            BCMGX_CHECK_LAUNCH();
+        };
+        if constexpr (sizeof(XT) == 4) {
+            if (sh.W == 4) {
+                go(k_blk_box<OP, 4, VT, XT, FT, MT, YT>);
+                return true;
+            }
+        }
+        if (sh.W == 2) go(k_blk_box<OP, 2, VT, XT, FT, MT, YT>);
+        else go(k_blk_box<OP, 1, VT, XT, FT, MT, YT>);
+        return true;
+    }
+    return false;
+}
+
+// A residual or a sweep on blocks of K columns of a level: the box kernel or the CSR one.
+template <int OP, typename VT, typename XT, typename FT, typename MT, typename YT>
+static void level_blk_rowop(const DevCsr& A, int K, const VT* val, const XT* x, const FT* f, const MT* M, YT* y,
+    const int* skip, cudaStream_t s)
+{
+    if (launch_blk_box<OP>(A, K, val, x, f, M, y, skip, s)) return;
+    launch_blk_rowop<OP>(A.n, A.m, K, K, A.row.p, A.col.p, val, x, f, M, y, 1.0, 0.0, skip, s);
+}
+
 // ------------------------------------------------------------------------------------------
 // the cycle: one code path for a single vector (lk < 0: the sub-warp row kernels above) and for
 // blocks of 2^lk right-hand sides (the block kernels of blockops.cuh)
@@ -774,7 +828,7 @@ struct Cycle {
             return;
         }
         if (lk < 0) launch_rowop_A<OP>(A.tpr, A, val, x, f, M, y, 1.0, 0.0, skip, s);
-        else launch_blk_rowop<OP>(A.n, A.m, 1 << lk, 1 << lk, A.row.p, A.col.p, val, x, f, M, y, 1.0, 0.0, skip, s);
+        else level_blk_rowop<OP>(A, 1 << lk, val, x, f, M, y, skip, s);
     }
     template <typename FT, typename MT, typename YT, typename CT>
     void first(int n, const FT* f, const MT* M, YT* u, CT* fcopy) const
@@ -1816,18 +1870,14 @@ void time_block_kernels(bcmgx_hierarchy* H, int K, int reps, double* out)
         y32.alloc(nk, s);
         fill_probe(x32.p, (long)nk, 1u, s);
         fill_probe(f32b.p, (long)nk, 2u, s);
-        out[0] = timeit([&] { launch_blk_rowop<OP_JACOBI>(A.n, A.m, kp, kp, A.row.p, A.col.p, A.val32.p,
-                                  (const float*)x32.p, (const float*)f32b.p, V.M32.p, y32.p, 1.0, 0.0, nullptr, s); });
-        out[1] = timeit([&] { launch_blk_rowop<OP_RESID>(A.n, A.m, kp, kp, A.row.p, A.col.p, A.val32.p,
-                                  (const float*)x32.p, (const float*)f32b.p, (const float*)nullptr, y32.p, 1.0, 0.0, nullptr, s); });
+        out[0] = timeit([&] { level_blk_rowop<OP_JACOBI>(A, kp, A.val32.p, (const float*)x32.p, (const float*)f32b.p, V.M32.p, y32.p, nullptr, s); });
+        out[1] = timeit([&] { level_blk_rowop<OP_RESID>(A, kp, A.val32.p, (const float*)x32.p, (const float*)f32b.p, (const float*)nullptr, y32.p, nullptr, s); });
         BCMGX_CUDA(cudaStreamSynchronize(s));
     } else {
         f.alloc(nk, s);
         fill_probe(f.p, (long)nk, 2u, s);
-        out[0] = timeit([&] { launch_blk_rowop<OP_JACOBI>(A.n, A.m, kp, kp, A.row.p, A.col.p, A.val.p,
-                                  (const double*)x.p, (const double*)f.p, V.M.p, y.p, 1.0, 0.0, nullptr, s); });
-        out[1] = timeit([&] { launch_blk_rowop<OP_RESID>(A.n, A.m, kp, kp, A.row.p, A.col.p, A.val.p,
-                                  (const double*)x.p, (const double*)f.p, (const double*)nullptr, y.p, 1.0, 0.0, nullptr, s); });
+        out[0] = timeit([&] { level_blk_rowop<OP_JACOBI>(A, kp, A.val.p, (const double*)x.p, (const double*)f.p, V.M.p, y.p, nullptr, s); });
+        out[1] = timeit([&] { level_blk_rowop<OP_RESID>(A, kp, A.val.p, (const double*)x.p, (const double*)f.p, (const double*)nullptr, y.p, nullptr, s); });
     }
     out[2] = timeit([&] { launch_blk_rowop<OP_AXPBY>(A.n, A.m, kp, kp, A.row.p, A.col.p, A.val.p, (const double*)x.p,
                               (const double*)nullptr, (const double*)nullptr, y.p, 1.0, 0.0, nullptr, s); });
@@ -2232,6 +2282,12 @@ static int finish_solve(bcmgx_hierarchy* H, bcmgx_solve_info* info, int n)
     return S.iter >= P.itnlim ? BCMGX_ERR_NO_CONVERGENCE : BCMGX_OK;
 }
 
+// Rows from which a hierarchy's first solve takes its graph: capturing, instantiating and destroying one
+// costs 0.5 to 1 ms of host time, which a solve of few and short iterations does not win back (set-up +
+// solve of 7-point 10^3 1.69 -> 1.43 ms without it, of 50^3 4.96 -> 4.55), while long solves are up to a
+// tenth shorter with it. Both drivers launch the same kernels and give the same iterates.
+constexpr int kGraphRows = 300000;
+
 // Flexible CG (FCG.cu:27-165) on device vectors b, x (x: x0 in, solution out).
 // Stream path: iterations are enqueued one ahead of the convergence test (the extra iteration skips
 // itself on the device once `done` is set), so the GPU never waits for the host between
@@ -2284,9 +2340,3 @@ int fcg_solve(bcmgx_hierarchy* H, const double* b, double* x, bcmgx_solve_info* 
 }
 
 }  // namespace bcmgx
-// Rows from which a hierarchy's first solve takes its graph: capturing, instantiating and destroying one
-// costs 0.5 to 1 ms of host time, which a solve of few and short iterations does not win back (set-up +
-// solve of 7-point 10^3 1.69 -> 1.43 ms without it, of 50^3 4.96 -> 4.55), while long solves are up to a
-// tenth shorter with it. Both drivers launch the same kernels and give the same iterates.
-constexpr int kGraphRows = 300000;
-
