@@ -303,14 +303,17 @@ struct BoxArgs {
     const unsigned char* form;
     const unsigned* mask;
 };
-constexpr int kBlkBoxP = 4;   // rows of a slot
+// rows of a slot: two with four blocks per SM in the sweeps and residuals (27-point 100^3, 32 columns: 148 us a
+// FP32 sweep, 155 with four rows and three blocks, 177 with four and two), four with two blocks in the
+// product with its dots (349 us; 357 with two and four)
+constexpr int kBlkBoxP = 2, kBlkBoxDotsP = 4;
 
 // As blk_rows, but a slot takes P rows s apart: they share the block rows of X that they gather (a plane's
 // P + 2 lines of three), so a row costs 9 (P + 2) / P vector loads instead of 27, and no entry is
 // staged. The entries of a row are added in CSR order; a block row of X is loaded when one of the P rows
 // has its column, and added to the rows that have it. Dynamic shared memory: 36 values a form. Bound by the
 // latency of the gathers at 32 columns (their block is larger than L2): FP32 sweeps of 27-point 100^3 take
-// 177 us instead of 217, with 8 columns 56 instead of 180, with 2 23 instead of 180.
+// 148 us instead of 217, with 8 columns 47 instead of 180, with 2 23 instead of 180.
 template <int W, int P, typename VT, typename XT, typename Epi>
 __device__ __forceinline__ void blk_box_rows(int n, int lpe_log2, int ld, int K, const BoxArgs& box,
     const VT* __restrict__ vals, const XT* __restrict__ X, Epi&& epi)
@@ -425,7 +428,7 @@ __device__ __forceinline__ void blk_box_rows(int n, int lpe_log2, int ld, int K,
 
 // the row operations of k_blk_rowop on a 27-point box
 template <int OP, int W, typename VT, typename XT, typename FT, typename MT, typename YT>
-__global__ void __launch_bounds__(kBlkRowopThreads, 2) k_blk_box(int n, int lpe_log2, int ld, int K, BoxArgs box,
+__global__ void __launch_bounds__(kBlkRowopThreads, 4) k_blk_box(int n, int lpe_log2, int ld, int K, BoxArgs box,
     const VT* __restrict__ vals, const XT* __restrict__ X, const FT* __restrict__ F, const MT* __restrict__ M,
     YT* __restrict__ Y, const int* __restrict__ skip)
 {
@@ -493,17 +496,17 @@ __global__ void k_blk_prolong(int n, int lk, const int* __restrict__ agg, const 
     }
 }
 
-// A box level's arguments, the items of its slots (kBlkBoxP rows each) and the table's bytes.
+// A box level's arguments, the items of its slots (P rows each) and the table's bytes.
 struct BoxLevel {
     BoxArgs box;
     long items;
     size_t smem;
 };
-inline BoxLevel box_level(const DevCsr& A, size_t value_bytes)
+inline BoxLevel box_level(const DevCsr& A, size_t value_bytes, int P)
 {
     BoxLevel b;
     b.box = BoxArgs { A.st_box, A.st_offs.o[4], A.st_offs.o[22], A.st_nform, A.st_form.p, A.st_mask.p };
-    const long ps = (long)kBlkBoxP * A.st_box;
+    const long ps = (long)P * A.st_box;
     b.items = ((long)A.n + ps - 1) / ps * A.st_box;
     b.smem = (size_t)A.st_nform * 36 * value_bytes;
     return b;

@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kBlkThreads, 2) k_blk_box_dots(int n, int lpe_
 {
     if (skip && *skip) return;
     double acc[3][W] = {};
-    blk_box_rows<W, kBlkBoxP>(n, lpe_log2, kp, kp, box, tab, PV, [&](long, long o, const double (&s)[W]) {
+    blk_box_rows<W, kBlkBoxDotsP>(n, lpe_log2, kp, kp, box, tab, PV, [&](long, long o, const double (&s)[W]) {
         double vi[W], ri[W], qi[W];
         stv<W>(PW + o, s);
         ldw<W>(PV + o, vi);
@@ -415,7 +415,7 @@ void launch_dots(const DevCsr& A, const MultiWork& wk, const double* pv, double*
     const int kp = 1 << wk.lk;
     if (A.stencil && A.st_box > 0 && A.st_tab64.p) {
         auto box = [&](auto kern) {
-            const BoxLevel bl = box_level(A, sizeof(double));
+            const BoxLevel bl = box_level(A, sizeof(double), kBlkBoxDotsP);
             ensure_smem_limit((const void*)kern, bl.smem);
             const long need = ceil_div(bl.items, kBlkThreads >> sh.lpe_log2);
             const int grid = (int)std::min<long>(std::max<long>(need, 1),

@@ -683,7 +683,7 @@ static bool launch_blk_box(const DevCsr& A, int K, const VT* val, const XT* x, c
         const BlkShape sh = blk_shape(K, (int)sizeof(XT));
         if (sh.W > 1 && (!aligned_for(x, sh.W, sizeof(XT)) || !aligned_for(y, sh.W, sizeof(YT)) || !aligned_for(f, sh.W, sizeof(FT))))
             return false;
-        const BoxLevel bl = box_level(A, sizeof(VT));
+        const BoxLevel bl = box_level(A, sizeof(VT), kBlkBoxP);
         auto go = [&](auto kern) {
             ensure_smem_limit((const void*)kern, bl.smem);
             const long need = ceil_div(bl.items, kBlkRowopThreads >> sh.lpe_log2);
