@@ -217,15 +217,16 @@ void scan_exclusive_dev(const int* in, int* out, long n, cudaStream_t s)
 // row to dpos (-1: none) and, when dcol is given, every column as an int16 offset from its row
 // (clamped; the caller keeps them only when the largest offset fits).
 // A block takes 256 consecutive rows: their columns, one contiguous range, go to shared memory with
-// asynchronous copies that are all in flight at once, then every lane walks its own row there, one
-// word in 32 skipped so that rows of 32 entries do not meet in one bank. The pass is then bound by
-// the column stream: on the 27-point 160^3 matrix (437 MB of columns) the checked product takes 415 us
-// instead of 910, 236 of them the product, where a warp per row took 655 us for the checks. Rows whose block holds more
+// asynchronous copies that are all in flight at once (16 bytes each where the array allows it, 4 at its
+// end), then every lane walks its own row there, 4 words in 128 skipped so that rows of 32 entries do not
+// all meet in one bank. The pass is then bound by
+// the column stream: on the 27-point 160^3 matrix (437 MB of columns) the checked product takes 385 us
+// (415 with 4-byte copies) instead of 910, 236 of them the product, where a warp per row took 655 us for the checks. Rows whose block holds more
 // than kValCap entries, or an offset out of order, are walked by a warp each from global memory.
 constexpr int kValRows = 256;
 constexpr int kValCap = 8192;
 
-__device__ __forceinline__ int val_slot(int j) { return j + (j >> 5); }
+__device__ __forceinline__ int val_slot(int j) { return j + ((j >> 7) << 2); }   // keeps 16-byte chunks whole
 
 template <bool OFFS>
 __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long nnz, const int* __restrict__ row,
@@ -233,8 +234,9 @@ __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long n
     int* __restrict__ dpos)
 {
     __shared__ int rows_s[kValRows + 1];
-    __shared__ int cols_s[kValCap + kValCap / 32];
+    __shared__ __align__(16) int cols_s[kValCap + kValCap / 32 + 8];
     const int tid = threadIdx.x, lane = tid & 31;
+    const bool wide = ((size_t)col & 15) == 0;
     int mx = 0, mo = 0, bad = 0;
     const long ntiles = ((long)n + kValRows - 1) / kValRows;
     for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -254,20 +256,26 @@ __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long n
             else mx = max(mx, e - b);
         }
         const bool all_ok = __syncthreads_and(ok);
-        const int b0 = rows_s[0];
+        const int b0 = rows_s[0], a0 = wide ? b0 & 3 : 0;   // cols_s starts at entry b0 - a0
         const long total = all_ok ? (long)rows_s[nr] - b0 : 0;   // the rows' ranges follow one another
         if (all_ok && total <= kValCap) {
-            for (int j = tid; j < (int)total; j += kValRows)
+            const int* src = col + (b0 - a0);
+            const int cnt = (int)total + a0, whole = wide ? cnt & ~3 : 0;
+            for (int j = 4 * tid; j < whole; j += 4 * kValRows)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(cols_s + val_slot(j))),
+                    "l"(src + j) : "memory");
+            for (int j = whole + tid; j < cnt; j += kValRows)
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(cols_s + val_slot(j))),
-                    "l"(col + b0 + j) : "memory");
+                    "l"(src + j) : "memory");
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
             __syncthreads();
             if (tid < nr) {
                 int prev = -1, d = -1;
-                for (int j = b - b0; j < e - b0; j++) {
+                const int j0 = b - b0 + a0, j1 = e - b0 + a0;
+                for (int j = j0; j < j1; j++) {
                     const int c = cols_s[val_slot(j)];
-                    if (c < 0 || c >= m) bad |= ERR_COLRANGE;
-                    if (j > b - b0 && prev >= c) bad |= ERR_COLSORT;
+                    if ((unsigned)c >= (unsigned)m) bad |= ERR_COLRANGE;
+                    if (j > j0 && prev >= c) bad |= ERR_COLSORT;
                     if (c == r) d = j;
                     if (OFFS) {
                         const int off = c - r;
@@ -277,11 +285,11 @@ __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long n
                     prev = c;
                 }
                 if (need_diag && d < 0) bad |= ERR_NODIAG;
-                if (OFFS && dpos) dpos[r] = d < 0 ? -1 : b0 + d;
+                if (OFFS && dpos) dpos[r] = d < 0 ? -1 : b0 - a0 + d;
             }
             if (OFFS && dcol) {
                 __syncthreads();
-                for (int j = tid; j < (int)total; j += kValRows) dcol[b0 + j] = (short)cols_s[val_slot(j)];
+                for (int j = tid; j < (int)total; j += kValRows) dcol[b0 + j] = (short)cols_s[val_slot(j + a0)];
             }
         } else {
             for (int i = tid >> 5; i < nr; i += kValRows / 32) {

@@ -43,12 +43,15 @@ def spoil(kind, row, col, n, r):
 SIZES = [(1, ()), (255, ()), (256, ()), (257, ()), (3000, (5, 6, 2999)), (3000, ())]
 
 
+@pytest.mark.parametrize("shift", [0, 1, 3])
 @pytest.mark.parametrize("n,dense", SIZES)
-def test_accepts(bx, cuda, n, dense):
+def test_accepts(bx, cuda, n, dense, shift):
+    """shift: the columns start that many words past a 16-byte boundary."""
     import torch
     row, col, val = tridiagonal(n, dense)
     x = np.random.default_rng(1).uniform(-1, 1, n)
-    t = [torch.from_numpy(a).to(cuda) for a in (row, col, val, x)]
+    t = [torch.from_numpy(a).to(cuda) for a in (row, np.concatenate([np.full(shift, -5, np.int32), col]), val, x)]
+    t[1] = t[1][shift:]
     y = bx.spmv(*t, torch.empty(n, dtype=torch.float64, device=cuda)).cpu().numpy()
     import scipy.sparse as sp
     want = sp.csr_matrix((val, col, row), shape=(n, n)) @ x
