@@ -2002,11 +2002,13 @@ __device__ __forceinline__ unsigned vc_hash(unsigned long long b)
 }
 
 // Inserts bit pattern b into a kVcSlots-slot set (linear probing): 1 when it was new, 0 when it was
-// there, -1 when the set is full.
+// there, -1 when kVcProbes slots are taken by others (a set of at most kValueCodes values is a quarter full
+// and has no runs that long; walking a full set in global memory took a collection of distinct values 240 us).
+constexpr int kVcProbes = 128;
 __device__ __forceinline__ int vc_insert(unsigned long long* keys, unsigned long long b)
 {
     unsigned h = vc_hash(b);
-    for (int probe = 0; probe < kVcSlots; probe++) {
+    for (int probe = 0; probe < kVcProbes; probe++) {
         const unsigned long long k = *(volatile unsigned long long*)(keys + h);
         if (k == b) return 0;
         if (k == kVcEmpty) {
@@ -2043,6 +2045,7 @@ __global__ void k_vc_collect(long nnz, const double* __restrict__ val, unsigned 
     for (int i = threadIdx.x; i < kVcSlots; i += blockDim.x) {
         const unsigned long long b = keys[i];
         if (b == kVcEmpty) continue;
+        if (*(volatile int*)over) return;
         const int r = vc_insert(gkeys, b);
         if (r < 0 || (r > 0 && atomicAdd(gcount, 1) >= kValueCodes)) atomicExch(over, 1);
     }
