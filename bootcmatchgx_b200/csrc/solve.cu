@@ -2076,10 +2076,35 @@ static void fcg_iteration(bcmgx_hierarchy* H, bool even, double* x, double* hist
     fcg_update(n, pv, od, x, pw, oq, r, st, part, hist, skip, s);
 }
 
-// Adds the whole solve of hierarchy H to graph g as an independent branch: the start-up, then a
-// WHILE conditional node whose body is two iterations (the second skips itself once the first
-// converges) followed by a kernel that sets the loop condition from the device-side `done` flag.
-// The branch works on the hierarchy's own b / x buffers (gb, gx).
+// Adds the FCG loop on x to graph g after the nodes `after`: a WHILE conditional node whose body is two
+// iterations (the second skips itself once the first converges) followed by a kernel that sets the
+// loop condition from the device-side `done` flag.
+static void add_loop_to_graph(bcmgx_hierarchy* H, cudaGraph_t g, const std::vector<cudaGraphNode_t>& after, double* x)
+{
+    cudaStream_t s = H->stream;
+    const long long c0 = launch_count();
+    cudaGraphConditionalHandle h;
+    BCMGX_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = h;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t wn;
+    BCMGX_CUDA(cudaGraphAddNode(&wn, g, after.data(), after.size(), &cp));
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    BCMGX_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    fcg_iteration(H, true, x, H->hist.p, &H->st.p->done);
+    fcg_iteration(H, false, x, H->hist.p, &H->st.p->done);
+    launch_dep<2>(k_set_while, 1, 1, 0, s, h, (const FcgState*)H->st.p);
+    BCMGX_CHECK_LAUNCH();
+    BCMGX_CUDA(cudaStreamEndCapture(s, &body));
+    H->graph_body_kernels = launch_count() - c0;
+    note_launches(-H->graph_body_kernels);   // captured, not launched
+}
+
+// Adds the whole solve of hierarchy H to graph g as an independent branch: the start-up, then the
+// loop. The branch works on the hierarchy's own b / x buffers (gb, gx).
 static void add_solve_to_graph(bcmgx_hierarchy* H, cudaGraph_t g)
 {
     cudaStream_t s = H->stream;
@@ -2100,27 +2125,9 @@ static void add_solve_to_graph(bcmgx_hierarchy* H, cudaGraph_t g)
     std::vector<cudaGraphNode_t> tail(deps, deps + ndeps);
     cudaGraph_t gg = g;
     BCMGX_CUDA(cudaStreamEndCapture(s, &gg));
-    const long long c1 = launch_count();
-    cudaGraphConditionalHandle h;
-    BCMGX_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t wn;
-    BCMGX_CUDA(cudaGraphAddNode(&wn, g, tail.data(), tail.size(), &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    BCMGX_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    fcg_iteration(H, true, H->gx.p, H->hist.p, &H->st.p->done);
-    fcg_iteration(H, false, H->gx.p, H->hist.p, &H->st.p->done);
-    launch_dep<2>(k_set_while, 1, 1, 0, s, h, (const FcgState*)H->st.p);
-    BCMGX_CHECK_LAUNCH();
-    BCMGX_CUDA(cudaStreamEndCapture(s, &body));
-    const long long c2 = launch_count();
-    H->graph_startup_kernels = c1 - c0;
-    H->graph_body_kernels = c2 - c1;
-    note_launches(-(c2 - c0));   // captured, not launched
+    H->graph_startup_kernels = launch_count() - c0;
+    note_launches(-H->graph_startup_kernels);   // captured, not launched
+    add_loop_to_graph(H, g, tail, H->gx.p);
 }
 
 static void build_solve_graph(bcmgx_hierarchy* H)
@@ -2132,11 +2139,14 @@ static void build_solve_graph(bcmgx_hierarchy* H)
     BCMGX_CUDA(cudaGraphDestroy(g));
 }
 
-// Kernels launched by one graph solve of H that ran `iters` iterations.
+// Kernels launched by the captured loop of H in `iters` iterations, and by a whole graph solve.
+static long long loop_launches(const bcmgx_hierarchy* H, int iters, int bad)
+{
+    return H->graph_body_kernels * std::max(1LL, (long long)(iters + 1) / 2 + (bad ? 1 : 0));
+}
 static long long graph_launches(const bcmgx_hierarchy* H, int iters, int bad)
 {
-    const long long bodies = std::max(1LL, (long long)(iters + 1) / 2 + (bad ? 1 : 0));
-    return H->graph_startup_kernels + H->graph_body_kernels * bodies;
+    return H->graph_startup_kernels + loop_launches(H, iters, bad);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2282,25 +2292,60 @@ static int finish_solve(bcmgx_hierarchy* H, bcmgx_solve_info* info, int n)
     return S.iter >= P.itnlim ? BCMGX_ERR_NO_CONVERGENCE : BCMGX_OK;
 }
 
-// Rows from which a hierarchy's first solve takes its graph: capturing, instantiating and destroying one
-// costs 0.5 to 1 ms of host time, which a solve of few and short iterations does not win back (set-up +
-// solve of 7-point 10^3 1.69 -> 1.43 ms without it, of 50^3 4.96 -> 4.55), while long solves are up to a
-// tenth shorter with it. Both drivers launch the same kernels and give the same iterates.
-constexpr int kGraphRows = 300000;
+// A hierarchy of fewer rows than kGraphRows starts its first solve without a graph: capturing,
+// instantiating and destroying one costs 0.4 to 0.7 ms of host time, which a solve of few and short
+// iterations does not win back. An iteration takes 17 us (1,000 rows) to 38 us (262,000) longer on the
+// stream than in a graph, so after kGraphLook iterations the residual's mean reduction says how many are
+// left, and where that is kGraphLeft or more (the loop's capture then costs less than they save) the rest
+// runs as a graph of the loop. Set-up + solve + free in ms with the graph from the start / by this rule / on
+// the stream alone: 7-point 10^3 (9 iterations) 1.85 / 1.57 / 1.55; 50^3 (22) 5.03 / 5.10 / 5.06, to 1e-12 (32)
+// 5.87 / 5.98 / 6.19; 27-point 64^3 (22) 8.37 / 8.36 / 8.57; diffusion 64^3 to 1e-12 (50) 11.2 / 11.6 / 12.3.
+// All drivers launch the same kernels and give the same iterates.
+constexpr int kGraphRows = 300000, kGraphLook = 3, kGraphLeft = 10;
+
+// Whether the solve in state S has at least kGraphLeft iterations to go.
+static bool graph_pays(const FcgState& S)
+{
+    if (S.itnlim - S.iter < kGraphLeft) return false;
+    const double l2 = std::sqrt(S.rnorm2);
+    if (!(l2 > 0.0) || !(S.tol > 0.0)) return true;
+    // per step, the start-up counted as one; no reduction so far: no end in sight
+    const double rate = std::log(S.delta0 / l2) / (S.iter + 1);
+    return !(rate > 0.0) || std::log(l2 / S.tol) >= kGraphLeft * rate;
+}
+
+// The rest of a solve on x whose first iterations, an even number of them, are in the stream.
+struct LoopGraph {
+    cudaGraphExec_t exec = nullptr;
+    void run(bcmgx_hierarchy* H, double* x)
+    {
+        cudaGraph_t g = nullptr;
+        BCMGX_CUDA(cudaGraphCreate(&g, 0));
+        add_loop_to_graph(H, g, {}, x);
+        BCMGX_CUDA(cudaGraphInstantiate(&exec, g, 0));
+        BCMGX_CUDA(cudaGraphDestroy(g));
+        BCMGX_CUDA(cudaGraphLaunch(exec, H->stream));
+    }
+    ~LoopGraph()
+    {
+        if (exec) cudaGraphExecDestroy(exec);
+    }
+};
 
 // Flexible CG (FCG.cu:27-165) on device vectors b, x (x: x0 in, solution out).
 // Stream path: iterations are enqueued one ahead of the convergence test (the extra iteration skips
 // itself on the device once `done` is set), so the GPU never waits for the host between
-// iterations. Graph path (use_graph, not with dispnorm): one launch of the captured solve.
+// iterations. Graph path (use_graph, not with dispnorm): one launch of the captured solve; a small
+// hierarchy's first solve starts on the stream (kGraphRows).
 int fcg_solve(bcmgx_hierarchy* H, const double* b, double* x, bcmgx_solve_info* info)
 {
     ensure_solve_workspace(H);
     cudaStream_t s = H->stream;
     const int n = H->lv[0].A.n;
     const bcmgx_params& P = H->prm;
-    // a small hierarchy's first solve goes without the graph (kGraphRows)
+    const bool graph = P.use_graph == 1 && !P.dispnorm;
     const bool first = H->solves++ == 0 && n < kGraphRows;
-    if (P.use_graph == 1 && !P.dispnorm && (H->iter_graph || !first)) {
+    if (graph && (H->iter_graph || !first)) {
         if (!H->iter_graph) build_solve_graph(H);
         BCMGX_CUDA(cudaMemcpyAsync(H->gb.p, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         BCMGX_CUDA(cudaMemcpyAsync(H->gx.p, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
@@ -2323,6 +2368,7 @@ int fcg_solve(bcmgx_hierarchy* H, const double* b, double* x, bcmgx_solve_info* 
         BCMGX_CUDA(cudaMemcpyAsync(ring + (k % 2), H->st.p, sizeof(FcgState), cudaMemcpyDeviceToHost, s));
         BCMGX_CUDA(cudaEventRecord(H->ev_it[k % 2], s));
     };
+    LoopGraph loop;
     enqueue(0);
     int k = 0;
     for (;;) {
@@ -2332,10 +2378,16 @@ int fcg_solve(bcmgx_hierarchy* H, const double* b, double* x, bcmgx_solve_info* 
         if (P.dispnorm && !S.bad) std::printf("%d) r norm: %.10lf\n", S.iter - 1, std::sqrt(S.rnorm2));
         if (S.done) break;
         k++;
+        // k + 1 iterations are in the stream, k of them have been looked at
+        if (graph && k >= kGraphLook && k % 2 == 1 && graph_pays(S)) {
+            loop.run(H, x);
+            break;
+        }
     }
     BCMGX_CUDA(cudaEventRecord(H->ev1, s));
     BCMGX_CUDA(cudaMemcpyAsync(H->st_host, H->st.p, sizeof(FcgState), cudaMemcpyDeviceToHost, s));
     BCMGX_CUDA(cudaStreamSynchronize(s));
+    if (loop.exec) note_launches(loop_launches(H, H->st_host->iter - (k + 1), H->st_host->bad));
     return finish_solve(H, info, n);
 }
 

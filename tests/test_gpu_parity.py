@@ -362,8 +362,8 @@ def test_cli_matches_golden(golden, cuda, tmp_path):
 @pytest.mark.parametrize("prec", ["FP64", "FP32"])
 def test_graph_and_stream_drivers_agree(bx, cuda, case, prec):
     """The graph-captured solve (WHILE conditional node) and the stream solve (one-iteration
-    lookahead) run the same kernels: identical iterations and identical solutions. A second solve
-    on the same hierarchy relaunches the captured graph."""
+    lookahead) run the same kernels: identical iterations and identical solutions. A small
+    hierarchy's first solve starts on the stream; its second is the captured one."""
     A = as_csr(bx, case)
     b = A @ np.random.default_rng(4).uniform(-1, 1, A.shape[0])
     out = {}
