@@ -38,6 +38,7 @@ constexpr int kChHalo = 8192;            // halo slots and push entries of a blo
 // Per block: sizes, and its arrays at rank * (cap) of the plan's buffers.
 struct ChainSizes {
     int entries, halo, push, slices, width;   // width: steps of the widest slice
+    int need[kChCtas];                        // halo slots by the block that owns their rows
 };
 
 template <typename T>
@@ -196,42 +197,55 @@ __global__ void __launch_bounds__(kChThreads, 1) k_chain_cluster(ChainArgs<T> a,
     }
 }
 
-// Builds the plan: one cluster, block `rank` for its own rows. halo: every block's halo columns
-// (kChHalo each). sizes[rank].entries is -1 when the block's part does not fit its buffers.
-template <typename T>
-__global__ void __launch_bounds__(kChThreads) k_chain_plan(int n, int R, int S, int ecap, int scap,
-    const int* __restrict__ row, const int* __restrict__ col, const T* __restrict__ val, T* __restrict__ pval,
-    unsigned short* __restrict__ pidx, unsigned* __restrict__ push, int* __restrict__ sptr, int* halo, ChainSizes* sizes)
-{
-    // bits: the columns of other blocks that this block's rows use; base: their count before each word
-    __shared__ unsigned bits[(kChCtas * (kChMaxRows + 1)) / 32];
-    __shared__ int base[(kChCtas * (kChMaxRows + 1)) / 32 + 1];
-    __shared__ int npush, bad;
-    const int rank = (int)cluster_rank(), ctas = (int)gridDim.x, tid = threadIdx.x;
-    const int r0 = rank * R, nr = max(0, min(R, n - r0));
-    const int words = (n + 31) / 32, rs = 32 / S, slices = (nr + rs - 1) / rs;
-    for (int i = tid; i < words; i += kChThreads) bits[i] = 0u;
-    if (tid == 0) npush = bad = 0;
-    __syncthreads();
-    for (int r = r0 + tid; r < r0 + nr; r += kChThreads)
-        for (int j = row[r]; j < row[r + 1]; j++) {
-            const int c = col[j];
-            if (c < r0 || c >= r0 + R) atomicOr(&bits[c >> 5], 1u << (c & 31));
-        }
-    __syncthreads();
-    if (tid < 32) {   // one warp scans the words' counts
-        int run = 0;
-        for (int w0 = 0; w0 < words; w0 += 32) {
-            const int w = w0 + tid, c = w < words ? __popc(bits[w]) : 0;
-            int x = c;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (tid >= o) x += y;
+// The halo columns of block `rank` in shared memory, by all its threads: the bits of the other blocks'
+// columns that its rows use (ascending: the halo's slots), their count before each word; returns it whole.
+struct ChainHalo {
+    unsigned bits[(kChCtas * (kChMaxRows + 1)) / 32];
+    int base[(kChCtas * (kChMaxRows + 1)) / 32 + 1];
+    __device__ __forceinline__ int build(int n, int R, int rank, const int* __restrict__ row, const int* __restrict__ col)
+    {
+        const int tid = threadIdx.x, words = (n + 31) / 32, r0 = rank * R, r1 = min(r0 + R, n);
+        for (int i = tid; i < words; i += kChThreads) bits[i] = 0u;
+        __syncthreads();
+        for (int r = r0 + tid; r < r1; r += kChThreads)
+            for (int j = row[r]; j < row[r + 1]; j++) {
+                const int c = col[j];
+                if (c < r0 || c >= r0 + R) atomicOr(&bits[c >> 5], 1u << (c & 31));
             }
-            if (w < words) base[w] = run + x - c;
-            run += __shfl_sync(0xffffffffu, x, 31);
+        __syncthreads();
+        if (tid < 32) {   // one warp scans the words' counts
+            int run = 0;
+            for (int w0 = 0; w0 < words; w0 += 32) {
+                const int w = w0 + tid, c = w < words ? __popc(bits[w]) : 0;
+                int x = c;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (tid >= o) x += y;
+                }
+                if (w < words) base[w] = run + x - c;
+                run += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (tid == 0) base[words] = run;
         }
-        // and the slices' widths
+        __syncthreads();
+        return base[words];
+    }
+    // halo columns below c: the slot of a column that is one
+    __device__ __forceinline__ int slot(int c) const { return base[c >> 5] + __popc(bits[c >> 5] & ((1u << (c & 31)) - 1u)); }
+    __device__ __forceinline__ int slots_below(int c, int n, int H) const { return c < n ? slot(c) : H; }
+};
+
+// The plan's sizes, a block of the grid for each of the cluster's: its slices' widths (sptr) and its halo.
+// Neither this nor k_chain_fill is a cluster: where none of the wanted size can run, set-up goes on without.
+__global__ void __launch_bounds__(kChThreads) k_chain_sizes(int n, int R, int S, int scap, const int* __restrict__ row,
+    const int* __restrict__ col, int* __restrict__ sptr, ChainSizes* sizes)
+{
+    __shared__ ChainHalo halo;
+    const int rank = blockIdx.x, tid = threadIdx.x;
+    const int r0 = rank * R, nr = max(0, min(R, n - r0)), rs = 32 / S, slices = (nr + rs - 1) / rs;
+    const int H = halo.build(n, R, rank, row, col);
+    if (tid < (int)gridDim.x) sizes[rank].need[tid] = halo.slots_below((tid + 1) * R, n, H) - halo.slots_below(tid * R, n, H);
+    if (tid < 32) {
         int at = 0, widest = 0;
         for (int t0 = 0; t0 < slices; t0 += 32) {
             const int t = t0 + tid;
@@ -254,56 +268,61 @@ __global__ void __launch_bounds__(kChThreads) k_chain_plan(int n, int R, int S, 
         widest = __reduce_max_sync(0xffffffffu, widest);
         if (tid == 0) {
             sptr[(size_t)rank * scap + slices] = at;
-            base[words] = run;
-            if (at > ecap || run > kChHalo) bad = 1;
-            sizes[rank] = ChainSizes { at, run, 0, slices, widest };
+            sizes[rank].entries = at;
+            sizes[rank].halo = H;
+            sizes[rank].slices = slices;
+            sizes[rank].width = widest;
         }
+    }
+}
+
+// The plan's entries and push lists, once the sizes are known to fit ecap and pcap a block.
+template <typename T>
+__global__ void __launch_bounds__(kChThreads) k_chain_fill(int n, int R, int S, int ecap, int pcap, int scap,
+    const int* __restrict__ row, const int* __restrict__ col, const T* __restrict__ val, const int* __restrict__ sptr,
+    T* __restrict__ pval, unsigned short* __restrict__ pidx, unsigned* __restrict__ push, ChainSizes* sizes)
+{
+    __shared__ ChainHalo halo;
+    __shared__ int at[kChCtas];
+    const int rank = blockIdx.x, tid = threadIdx.x;
+    const int r0 = rank * R, nr = max(0, min(R, n - r0)), rs = 32 / S, slices = (nr + rs - 1) / rs;
+    const int H = halo.build(n, R, rank, row, col);
+    // An owner's list goes by the block that needs the value and by its slot there, so that consecutive
+    // threads store to consecutive addresses of one block (scattered, an FP64 solve of 127x93x75 rows took 2.4 %
+    // longer). at[own]: where the owner's list has this block's slots, less the first of them.
+    if (tid < (int)gridDim.x) {
+        int o = 0, all = 0;
+        for (int c = 0; c < (int)gridDim.x; c++) {
+            if (c == rank) o = all;
+            all += sizes[c].need[tid];
+        }
+        at[tid] = o - halo.slots_below(tid * R, n, H);
+        if (tid == rank) sizes[rank].push = all;
     }
     __syncthreads();
-    const int H = base[words];
-    if (!bad) {
-        for (int w = tid; w < words; w += kChThreads) {
-            unsigned m = bits[w];
-            for (int o = base[w]; m; o++, m &= m - 1u) halo[(size_t)rank * kChHalo + o] = 32 * w + __ffs((int)m) - 1;
-        }
-        for (int t = tid >> 5; t < slices; t += kChThreads / 32) {
-            const int lane = tid & 31, r = t * rs + lane / S;
-            const int b = r < nr ? row[r0 + r] : 0, e = r < nr ? row[r0 + r + 1] : 0;
-            const int o = sptr[(size_t)rank * scap + t], kk = (sptr[(size_t)rank * scap + t + 1] - o) / 32;
-            for (int q = 0; q < kk; q++) {
-                const int j = b + q * S + (lane & (S - 1));
-                int ix = R + H;
-                T v = T(0);
-                if (j < e) {
-                    const int c = col[j];
-                    v = val[j];
-                    ix = c >= r0 && c < r0 + R ? c - r0 : R + base[c >> 5] + __popc(bits[c >> 5] & ((1u << (c & 31)) - 1u));
-                }
-                pval[(size_t)rank * ecap + o + 32 * q + lane] = v;
-                pidx[(size_t)rank * ecap + o + 32 * q + lane] = (unsigned short)ix;
-            }
+    for (int w = tid; w < (n + 31) / 32; w += kChThreads) {
+        unsigned m = halo.bits[w];
+        for (int slot = halo.base[w]; m; slot++, m &= m - 1u) {
+            const int c = 32 * w + __ffs((int)m) - 1, own = c / R;
+            push[(size_t)own * pcap + at[own] + slot] = (unsigned)(c - own * R) | ((unsigned)rank << 11) | ((unsigned)slot << 15);
         }
     }
-    __threadfence();
-    cluster_arrive();
-    cluster_wait();
-    // the rows of this block in the other blocks' halos
-    for (int c = 0; c < ctas; c++) {
-        if (c == rank) continue;
-        const int hc = min(__ldcg(&sizes[c].halo), kChHalo);
-        for (int i = tid; i < hc; i += kChThreads) {
-            const int g = __ldcg(halo + (size_t)c * kChHalo + i);
-            if (g >= r0 && g < r0 + nr) {
-                const int p = atomicAdd(&npush, 1);
-                if (p < kChHalo) push[(size_t)rank * kChHalo + p] = (unsigned)(g - r0) | ((unsigned)c << 11) | ((unsigned)i << 15);
+    for (int t = tid >> 5; t < slices; t += kChThreads / 32) {
+        const int lane = tid & 31, r = t * rs + lane / S;
+        const int b = r < nr ? row[r0 + r] : 0, e = r < nr ? row[r0 + r + 1] : 0;
+        const int o = sptr[(size_t)rank * scap + t], kk = (sptr[(size_t)rank * scap + t + 1] - o) / 32;
+        for (int q = 0; q < kk; q++) {
+            const int j = b + q * S + (lane & (S - 1));
+            int ix = R + H;
+            T v = T(0);
+            if (j < e) {
+                const int c = col[j];
+                v = val[j];
+                ix = c >= r0 && c < r0 + R ? c - r0 : R + halo.slot(c);
             }
+            pval[(size_t)rank * ecap + o + 32 * q + lane] = v;
+            pidx[(size_t)rank * ecap + o + 32 * q + lane] = (unsigned short)ix;
         }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        if (npush > kChHalo) bad = 1;
-        sizes[rank].push = npush;
-        if (bad) sizes[rank].entries = -1;
     }
 }
 
@@ -371,36 +390,33 @@ static bool build_chain_t(Level& V, const T* val, cudaStream_t s)
     P->S = S;
     P->f32 = sizeof(T) == 4;
     if (P->R > kChMaxRows) return false;
+    // more slices than the warps hold: known before anything is launched
+    if (ceil_div(P->R, 32 / S) > kChWarps * kChSlices) return false;
     P->ecap = kChSmem / (int)(sizeof(T) + 2) / 32 * 32;
     P->scap = (P->R * S / 32 + 2 + 3) / 4 * 4 + 4;
-    DBuf<int> halo;
     P->val.alloc((size_t)ctas * P->ecap * sizeof(T), s);
     P->idx.alloc((size_t)ctas * P->ecap, s);
     P->push.alloc((size_t)ctas * kChHalo, s);
     P->sptr.alloc((size_t)ctas * P->scap, s);
     P->sizes.alloc((size_t)ctas * (sizeof(ChainSizes) / sizeof(int)), s);
-    halo.alloc((size_t)ctas * kChHalo, s);
-    {
-        cudaLaunchAttribute at[1];
-        auto kern = k_chain_plan<T>;
-        cudaLaunchConfig_t cfg = cluster_config(kern, ctas, 0, s, at);
-        note_launch();
-        BCMGX_CUDA(cudaLaunchKernelEx(&cfg, kern, n, P->R, S, P->ecap, P->scap, (const int*)A.row.p, (const int*)A.col.p,
-            val, (T*)P->val.p, P->idx.p, P->push.p, P->sptr.p, halo.p, (ChainSizes*)P->sizes.p));
-    }
+    ChainSizes* const sizes = (ChainSizes*)P->sizes.p;
+    note_launch();
+    k_chain_sizes<<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->scap, A.row.p, A.col.p, P->sptr.p, sizes);
+    BCMGX_CHECK_LAUNCH();
     ChainSizes z[kChCtas];
-    BCMGX_CUDA(cudaMemcpyAsync(z, P->sizes.p, sizeof(ChainSizes) * ctas, cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaMemcpyAsync(z, sizes, sizeof(ChainSizes) * ctas, cudaMemcpyDeviceToHost, s));
     BCMGX_CUDA(cudaStreamSynchronize(s));
     int E = 0, H = 0, N = 0, W = 0;
     for (int c = 0; c < ctas; c++) {
-        if (z[c].entries < 0) return false;
+        int push = 0;
+        for (int b = 0; b < ctas; b++) push += z[b].need[c];
+        if (z[c].entries > P->ecap || z[c].halo > kChHalo || push > kChHalo) return false;
         E = std::max(E, z[c].entries);
         H = std::max(H, z[c].halo);
         N = std::max(N, z[c].slices);
         W = std::max(W, z[c].width);
     }
     P->ns = (N + kChWarps - 1) / kChWarps;
-    if (P->ns > kChSlices) return false;
     // shared memory: both iterates (own rows, halo, the zero slot), f, M, and the entries of levels
     // with rows longer than the registers hold
     auto up16 = [](size_t b) { return (b + 15) / 16 * 16; };
@@ -430,6 +446,10 @@ static bool build_chain_t(Level& V, const T* val, cudaStream_t s)
         }
     });
     if (fit < 1) return false;
+    note_launch();
+    k_chain_fill<T><<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->ecap, kChHalo, P->scap, A.row.p, A.col.p, val, P->sptr.p,
+        (T*)P->val.p, P->idx.p, P->push.p, sizes);
+    BCMGX_CHECK_LAUNCH();
     V.chain = std::move(P);
     return true;
 }

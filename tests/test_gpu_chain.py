@@ -1,9 +1,14 @@
 """Sweep chains of small levels in one thread-block cluster (chain.cu) against one launch per sweep
 (BCMGX_CHAIN=0): the same rows, order of additions and update, so cycles and solves agree bit for bit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
 
+from conftest import ROOT
 from test_gpu_parity import fcg
 from test_gpu_staged import matrix
 
@@ -72,3 +77,57 @@ def test_chain_cycles(bx, cuda, monkeypatch, kw):
     v0, x0, i0, _ = cycle_and_solve(bx, monkeypatch, A, "0", **kw)
     v1, x1, i1, _ = cycle_and_solve(bx, monkeypatch, A, "1", **kw)
     assert np.array_equal(v0, v1) and i0["niter"] == i1["niter"] and np.array_equal(x0, x1)
+
+
+# The CUDA runtime's calls that a context without room for a cluster of more than 8 blocks answers with an error:
+# the launch and the occupancy query. Everything else goes to the runtime.
+NO_LARGE_CLUSTER = r"""
+#include <cuda_runtime_api.h>
+#include <dlfcn.h>
+static unsigned blocks(const cudaLaunchConfig_t* c)
+{
+    for (unsigned i = 0; c && i < c->numAttrs; i++)
+        if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) return c->attrs[i].val.clusterDim.x;
+    return 1;
+}
+static void* next(const char* name) { return dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), name); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a)
+{
+    if (blocks(c) > 8) return cudaErrorInvalidConfiguration;
+    return ((cudaError_t(*)(const cudaLaunchConfig_t*, const void*, void**))next("cudaLaunchKernelExC"))(c, f, a);
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* f, const cudaLaunchConfig_t* c)
+{
+    if (blocks(c) > 8) { *n = 0; return cudaSuccess; }
+    return ((cudaError_t(*)(int*, const void*, const cudaLaunchConfig_t*))next("cudaOccupancyMaxActiveClusters"))(n, f, c);
+}
+"""
+
+CHILD = r"""
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import bootcmatchgx_b200 as bx
+row, col, val = bx.laplacian_3d(27, 23, 21, 19)
+h = bx.prec_setup(row, col, val, bx.params_default(solver="FCG", preconditioner="BCMG", dispnorm=0, rtol=1e-8))
+c0 = bx.lib().bcmgx_launch_count()
+x, info = h.solve(np.random.default_rng(3).uniform(-1, 1, row.size - 1))
+print(info["status"], info["niter"], bx.lib().bcmgx_launch_count() - c0, x.tobytes().hex())
+"""
+
+
+def test_no_large_cluster(cuda, tmp_path):
+    """Where no cluster of 16 blocks can run, set-up succeeds and the level keeps one launch per sweep."""
+    src, lib = tmp_path / "fake.c", tmp_path / "fake.so"
+    src.write_text(NO_LARGE_CLUSTER)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-I/usr/local/cuda/include", str(src), "-o", str(lib), "-ldl"], check=True)
+
+    def child(**env):
+        e = {k: v for k, v in os.environ.items() if k not in ("BCMGX_CHAIN", "BCMGX_TPR")}
+        r = subprocess.run([sys.executable, "-c", CHILD, ROOT], env={**e, **env}, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return r.stdout.split()
+
+    launches, without, with_chain = child(BCMGX_CHAIN="0"), child(LD_PRELOAD=str(lib)), child()
+    assert without == launches and launches[0] == "0"
+    assert int(with_chain[2]) < int(launches[2])   # the level has a chain of 16 blocks where it may
