@@ -146,8 +146,8 @@ void pinned_free(void* p)
     g_pin_free.emplace(b, p);
 }
 
-// Builds one hierarchy (the body of bcmgx_setup). own_stream forces a library-owned stream even
-// when params name one (batch set-ups run concurrently, one stream each).
+// Builds one hierarchy (the body of bcmgx_setup). member: it is one of a batch, with a library-owned
+// stream even when params name one (batch set-ups run concurrently, one stream each).
 // Device-resident inputs are written by the caller's own work, normally on the legacy default
 // stream (torch's default stream, plain cudaMemcpy). A library-owned stream is non-blocking and
 // does not wait for that stream by itself, so every entry that reads caller buffers on it first
@@ -163,7 +163,7 @@ static void after_caller(cudaStream_t s, cudaEvent_t ev, bool own)
 // The row kernel of every level: BCMGX_TPR forces the codes (one code for every level, "-2", or
 // one per level, "-2,-2,4"; levels past the list take its last code); else the autotuner times
 // them (levels of at least 20,000 rows) or the default threads per row apply.
-void choose_level_kernels(bcmgx_hierarchy* H)
+void choose_level_kernels(bcmgx_hierarchy* H, bool chains)
 {
     const bcmgx_params* p = &H->prm;
     std::vector<int> force;
@@ -223,12 +223,25 @@ void choose_level_kernels(bcmgx_hierarchy* H)
         // 3,300 rows: 34.5 us with 4, 31 with 2, 35 with 1; of 7,900 rows: 73, 57, 54)
         const int tpr = V.A.tpr;
         if (force.empty() && tpr == 4 && !(p->autotune && V.A.n >= kTuneMinRows)) V.A.tpr = 2;
-        build_chain(V, f32, k, H->stream);
-        if (!V.chain) V.A.tpr = tpr;
+        if (chain_wanted(V.A, f32, k)) V.plain_tpr = tpr;
+        else V.A.tpr = tpr;
+    }
+    if (chains) plan_chains(H);
+}
+
+void plan_chains(bcmgx_hierarchy* H, bool fill)
+{
+    const int L = (int)H->lv.size();
+    for (int l = 0; l < L; l++) {
+        Level& V = H->lv[l];
+        if (!V.plain_tpr) continue;
+        const bool fits = build_chain(V, H->prm.vcycle_precision == BCMGX_VCYCLE_FP32 && l < L - 1, fill, H->stream);
+        if (!fits) V.A.tpr = V.plain_tpr;
+        if (fill || !fits) V.plain_tpr = 0;
     }
 }
 
-static bcmgx_hierarchy* setup_one(const bcmgx_csr* A, const bcmgx_params* p, int device, bool own_stream)
+static bcmgx_hierarchy* setup_one(const bcmgx_csr* A, const bcmgx_params* p, int device, bool member)
 {
     check_params(p);
     BCMGX_REQUIRE(A->n > 0 && A->n == A->m, BCMGX_ERR_INVALID_INPUT, "matrix must be square with n > 0");
@@ -242,7 +255,7 @@ static bcmgx_hierarchy* setup_one(const bcmgx_csr* A, const bcmgx_params* p, int
     H->device = dev;
     H->prm.device = dev;
     DeviceScope ds(dev);
-    if (p->stream && !own_stream) {
+    if (p->stream && !member) {
         H->stream = (cudaStream_t)p->stream;
     } else {
         BCMGX_CUDA(cudaStreamCreateWithFlags(&H->stream, cudaStreamNonBlocking));
@@ -265,7 +278,7 @@ static bcmgx_hierarchy* setup_one(const bcmgx_csr* A, const bcmgx_params* p, int
     BCMGX_CUDA(cudaEventRecord(t0.e, H->stream));
     stage_fault_init();
     build_hierarchy(H.get(), A);
-    choose_level_kernels(H.get());
+    choose_level_kernels(H.get(), !member);
     BCMGX_CUDA(cudaEventRecord(t1.e, H->stream));
     BCMGX_CUDA(cudaEventSynchronize(t1.e));
     float ms = 0;
@@ -465,6 +478,10 @@ int bcmgx_batch_get_hierarchy(bcmgx_batch* B, int k, bcmgx_hierarchy** h)
 {
     return guarded([&] {
         BCMGX_REQUIRE(B && h && k >= 0 && k < (int)B->hs.size(), BCMGX_ERR_INVALID_INPUT, "bad argument");
+        static std::mutex mu;
+        std::lock_guard<std::mutex> g(mu);
+        DeviceScope ds(B->device);
+        plan_chains(B->hs[k]);   // the caller may solve with it alone
         *h = B->hs[k];
     });
 }

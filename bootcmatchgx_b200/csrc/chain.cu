@@ -43,7 +43,7 @@ struct ChainSizes {
 
 template <typename T>
 struct ChainArgs {
-    int n, R, ecap, scap;
+    int n, R, ecap, pcap, scap;
     const ChainSizes* sizes;
     const T* val;                  // entries of the slices: lane l of step k of slice s at sptr[s] + 32 k + l
     const unsigned short* idx;     // their local columns
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kChThreads, 1) k_chain_cluster(ChainArgs<T> a,
     // address in the other block's first buffer
     int prow[kChPush];
     unsigned padr[kChPush];
-    const unsigned* gp = a.push + (size_t)rank * kChHalo;
+    const unsigned* gp = a.push + (size_t)rank * a.pcap;
     const unsigned xa = (unsigned)__cvta_generic_to_shared(x0) + (unsigned)(a.R * (int)sizeof(T));
     auto push_addr = [&](unsigned w) { return map_cta(xa + (w >> 15) * (unsigned)sizeof(T), (w >> 11) & 15u); };
 #pragma unroll
@@ -373,7 +373,7 @@ static void with_chain_kernel(int S, int ns, int st, F&& go)
 }
 
 template <typename T>
-static bool build_chain_t(Level& V, const T* val, cudaStream_t s)
+static bool build_chain_t(Level& V, const T* val, bool fill, cudaStream_t s)
 {
     const DevCsr& A = V.A;
     const int n = A.n, S = A.tpr;
@@ -392,11 +392,7 @@ static bool build_chain_t(Level& V, const T* val, cudaStream_t s)
     if (P->R > kChMaxRows) return false;
     // more slices than the warps hold: known before anything is launched
     if (ceil_div(P->R, 32 / S) > kChWarps * kChSlices) return false;
-    P->ecap = kChSmem / (int)(sizeof(T) + 2) / 32 * 32;
     P->scap = (P->R * S / 32 + 2 + 3) / 4 * 4 + 4;
-    P->val.alloc((size_t)ctas * P->ecap * sizeof(T), s);
-    P->idx.alloc((size_t)ctas * P->ecap, s);
-    P->push.alloc((size_t)ctas * kChHalo, s);
     P->sptr.alloc((size_t)ctas * P->scap, s);
     P->sizes.alloc((size_t)ctas * (sizeof(ChainSizes) / sizeof(int)), s);
     ChainSizes* const sizes = (ChainSizes*)P->sizes.p;
@@ -410,7 +406,8 @@ static bool build_chain_t(Level& V, const T* val, cudaStream_t s)
     for (int c = 0; c < ctas; c++) {
         int push = 0;
         for (int b = 0; b < ctas; b++) push += z[b].need[c];
-        if (z[c].entries > P->ecap || z[c].halo > kChHalo || push > kChHalo) return false;
+        if (z[c].entries > kChSmem / (int)(sizeof(T) + 2) || z[c].halo > kChHalo || push > kChHalo) return false;
+        P->pcap = std::max(P->pcap, push);
         E = std::max(E, z[c].entries);
         H = std::max(H, z[c].halo);
         N = std::max(N, z[c].slices);
@@ -446,29 +443,33 @@ static bool build_chain_t(Level& V, const T* val, cudaStream_t s)
         }
     });
     if (fit < 1) return false;
+    if (!fill) return true;
+    P->ecap = E;   // whole slices: every block's entries start on a 16-byte boundary
+    P->val.alloc((size_t)ctas * E * sizeof(T), s);
+    P->idx.alloc((size_t)ctas * E, s);
+    P->push.alloc((size_t)ctas * P->pcap, s);
     note_launch();
-    k_chain_fill<T><<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->ecap, kChHalo, P->scap, A.row.p, A.col.p, val, P->sptr.p,
+    k_chain_fill<T><<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->ecap, P->pcap, P->scap, A.row.p, A.col.p, val, P->sptr.p,
         (T*)P->val.p, P->idx.p, P->push.p, sizes);
     BCMGX_CHECK_LAUNCH();
     V.chain = std::move(P);
     return true;
 }
 
-void build_chain(Level& V, bool f32, int k, cudaStream_t s)
+bool chain_wanted(const DevCsr& A, bool f32, int k)
 {
-    V.chain.reset();
     const char* env = std::getenv("BCMGX_CHAIN");
-    if (env && env[0] == '0') return;
+    if ((env && env[0] == '0') || !chain_pays(A, k)) return false;
+    if (A.stencil || A.sliced || A.staged) return false;   // levels tuned to stream over the whole GPU
+    if (A.n <= 0 || A.m != A.n || A.n > kChCtas * kChMaxRows || A.tpr > 16) return false;
+    return A.nnz * (int64_t)((f32 ? 4 : 8) + 2) <= (int64_t)kChCtas * kChSmem;
+}
+
+bool build_chain(Level& V, bool f32, bool fill, cudaStream_t s)
+{
     const DevCsr& A = V.A;
-    if (!chain_pays(A, k)) return;
-    if (A.stencil || A.sliced || A.staged) return;   // levels tuned to stream over the whole GPU
-    if (A.n <= 0 || A.m != A.n || A.n > kChCtas * kChMaxRows || A.tpr > 16) return;
-    if (A.nnz * (int64_t)((f32 ? 4 : 8) + 2) > (int64_t)kChCtas * kChSmem) return;
-    if (f32) {
-        if (A.val32.p) build_chain_t<float>(V, A.val32.p, s);
-    } else {
-        build_chain_t<double>(V, A.val.p, s);
-    }
+    if (f32) return A.val32.p && build_chain_t<float>(V, A.val32.p, fill, s);
+    return build_chain_t<double>(V, A.val.p, fill, s);
 }
 
 template <typename T>
@@ -479,6 +480,7 @@ static void run_chain_t(const Level& V, const T* M, int k, const T* f, const T* 
     a.n = P.n;
     a.R = P.R;
     a.ecap = P.ecap;
+    a.pcap = P.pcap;
     a.scap = P.scap;
     a.sizes = (const ChainSizes*)P.sizes.p;
     a.val = (const T*)P.val.p;

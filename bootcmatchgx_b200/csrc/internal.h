@@ -224,7 +224,7 @@ void release_stencil(DevCsr& A);
 // A small level's sweep chains as one cluster launch (chain.cu): ctas blocks of R rows, the level's
 // entries by block and slice, the lists of values that blocks exchange, the shared-memory layout.
 struct ChainPlan {
-    int ctas = 0, n = 0, R = 0, S = 0, ns = 0, st = 0, ecap = 0, scap = 0;
+    int ctas = 0, n = 0, R = 0, S = 0, ns = 0, st = 0, ecap = 0, pcap = 0, scap = 0;
     bool f32 = false;
     size_t smem = 0;
     int off_f = 0, off_M = 0, off_x1 = 0, off_val = -1, off_idx = -1;
@@ -249,6 +249,7 @@ struct Level {
     DBuf<double> rhs, x, x2;
     DBuf<float> rhs32, x32, x232;
     std::unique_ptr<ChainPlan> chain;   // null: one launch per sweep
+    int plain_tpr = 0;   // a chain is wanted and not planned yet (plan_chains): A.tpr where there is none
 };
 
 struct SweepRecord {
@@ -491,11 +492,18 @@ inline void ensure_smem_limit(void (*kernel)(A...), size_t bytes)
 constexpr int kTuneMinRows = 20000;   // rows of the smallest level that the autotuner times
 // need64: see build_stencil
 int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s);
-void choose_level_kernels(bcmgx_hierarchy* H);
-// Sweep chains of a small level in one cluster (chain.cu): the plan (one host round trip; none when
-// the level does not fit, its longest chain of k sweeps is better as launches, or BCMGX_CHAIN=0), and k
+// chains: also plan the coarse sweep chains (plan_chains).
+void choose_level_kernels(bcmgx_hierarchy* H, bool chains = true);
+// Plans the chains of H's levels that are wanted and not planned yet; without fill only the levels whose
+// chain does not fit are settled (Level::plain_tpr). The members of a batch go without plans: their sweeps
+// run on the union's levels or in one block (Cycle::chain_in_block), there with the threads per row that
+// the hierarchy has on its own.
+void plan_chains(bcmgx_hierarchy* H, bool fill = true);
+// Sweep chains of a small level in one cluster (chain.cu): whether the level's longest chain, of k sweeps,
+// is for one (BCMGX_CHAIN=0: none is), whether it fits and with fill its plan (one host round trip), and k
 // sweeps from src (null: zero) into dst in the level's precision; false when they are not for a cluster.
-void build_chain(Level& V, bool f32, int k, cudaStream_t s);
+bool chain_wanted(const DevCsr& A, bool f32, int k);
+bool build_chain(Level& V, bool f32, bool fill, cudaStream_t s);
 bool run_chain(const Level& V, bool f32, int k, const void* f, const void* src, void* dst, const int* skip, cudaStream_t s);
 void stage_fault_init();
 void stage_fault_check();

@@ -2206,6 +2206,7 @@ void batch_build(bcmgx_batch* B)
     BCMGX_CUDA(cudaGraphCreate(&g, 0));
     for (bcmgx_hierarchy* H : B->hs) {
         ensure_solve_workspace(H);
+        plan_chains(H, false);
         BatchCaptureMode mode(H);
         add_solve_to_graph(H, g);
     }

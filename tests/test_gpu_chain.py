@@ -9,6 +9,8 @@ import pytest
 import scipy.sparse as sp
 
 from conftest import ROOT
+from test_gpu_batch import _systems
+from test_gpu_faults import pool_used_bytes
 from test_gpu_parity import fcg
 from test_gpu_staged import matrix
 
@@ -77,6 +79,50 @@ def test_chain_cycles(bx, cuda, monkeypatch, kw):
     v0, x0, i0, _ = cycle_and_solve(bx, monkeypatch, A, "0", **kw)
     v1, x1, i1, _ = cycle_and_solve(bx, monkeypatch, A, "1", **kw)
     assert np.array_equal(v0, v1) and i0["niter"] == i1["niter"] and np.array_equal(x0, x1)
+
+
+def test_plan_memory(bx, cuda, monkeypatch):
+    """A plan holds its level's entries (10 bytes each, rows padded to a slice's longest and blocks to the widest),
+    lists of what blocks exchange and nothing more: at most 64 bytes for an entry of the coarse levels."""
+    import torch
+    row, col, val = bx.laplacian_3d(7, 24, 24, 24)
+    p = fcg(bx, rtol=1e-8, autotune=0)
+    held, entries = [], 0
+    for chain in ("0", "0", "1"):   # (the first set-up fills the process-wide caches)
+        monkeypatch.setenv("BCMGX_CHAIN", chain)
+        torch.cuda.synchronize()
+        base = pool_used_bytes()
+        h = bx.prec_setup(row, col, val, p)
+        torch.cuda.synchronize()
+        held.append(pool_used_bytes() - base)
+        entries = sum(h.info()["nnz"][1:])
+        h.free()
+    assert 0 < held[2] - held[1] <= 64 * entries
+
+
+def test_batch_members_have_no_plans(bx, cuda, monkeypatch):
+    """A batch's members take no memory for chains that its solves never run, and one handed out to be solved
+    alone has them."""
+    import torch
+    systems = _systems(bx, 12, 4)
+    b = torch.from_numpy(np.random.default_rng(5).uniform(-1, 1, systems[3][0].size - 1)).to(cuda)
+    held, launches, xs = [], [], []
+    for chain in ("0", "0", "1"):
+        monkeypatch.setenv("BCMGX_CHAIN", chain)
+        torch.cuda.synchronize()
+        base = pool_used_bytes()
+        B = bx.Batch(systems, fcg(bx, rtol=1e-8), nthreads=4)
+        torch.cuda.synchronize()
+        held.append(pool_used_bytes() - base)
+        c0 = bx.lib().bcmgx_launch_count()
+        x, info = B.hierarchy(3).solve(b)
+        launches.append(bx.lib().bcmgx_launch_count() - c0)
+        xs.append((info["niter"], x.cpu().numpy()))
+        B.free()
+    assert held[2] == held[1]
+    assert launches[2] < launches[1]
+    # two threads per row instead of four: sums in another order
+    assert xs[2][0] == xs[1][0] and np.linalg.norm(xs[2][1] - xs[1][1]) <= 1e-8 * np.linalg.norm(xs[1][1])
 
 
 # The CUDA runtime's calls that a context without room for a cluster of more than 8 blocks answers with an error:
