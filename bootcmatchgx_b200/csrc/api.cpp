@@ -26,6 +26,12 @@ struct FailAllocScope {
     ~FailAllocScope() { t_fail_alloc_countdown = 0; }
 };
 
+FormAllocScope::FormAllocScope()
+{
+    const char* e = std::getenv("BCMGX_TEST_FAIL_FORM");
+    t_fail_alloc_countdown = (e && *e) ? std::max(0LL, std::atoll(e)) : 0;
+}
+
 // A CUDA event owned for the duration of a scope.
 struct ScopedEvent {
     cudaEvent_t e = nullptr;
@@ -188,7 +194,8 @@ void choose_level_kernels(bcmgx_hierarchy* H, bool chains)
         // negative: the staged kernel with -code threads per row (1, 2, 4 or 8); kSlicedCode: the
         // sliced kernel (one lane per row: the CSR kernels stand in for it with 1 thread per row)
         if (code == kStencilCode) {
-            build_stencil(V.A, l == 0 || !f32, H->stream);
+            const bool room = optional_form([&] { build_stencil(V.A, l == 0 || !f32, H->stream); });
+            if (!room) release_stencil(V.A);
             V.A.stencil = V.A.st_form.p != nullptr;
             if (V.A.stencil) {
                 release_sliced(V.A);
@@ -197,8 +204,9 @@ void choose_level_kernels(bcmgx_hierarchy* H, bool chains)
                 continue;
             }
             // a level that has no stencil form (a forced code, or a matrix of the same size as the one
-            // the code was tuned on): the sliced kernels, which take any level
-            code = kSlicedCode;
+            // the code was tuned on): the sliced kernels, which take any level; without room for the
+            // form the plain ones, which need none and add a row's entries in the same order
+            code = room ? kSlicedCode : 1;
         }
         release_stencil(V.A);
         if (code == kSlicedCode) {
@@ -235,7 +243,9 @@ void plan_chains(bcmgx_hierarchy* H, bool fill)
     for (int l = 0; l < L; l++) {
         Level& V = H->lv[l];
         if (!V.plain_tpr) continue;
-        const bool fits = build_chain(V, H->prm.vcycle_precision == BCMGX_VCYCLE_FP32 && l < L - 1, fill, H->stream);
+        const bool f32 = H->prm.vcycle_precision == BCMGX_VCYCLE_FP32 && l < L - 1;
+        bool fits = false;
+        optional_form([&] { fits = build_chain(V, f32, fill, H->stream); });
         if (!fits) V.A.tpr = V.plain_tpr;
         if (fill || !fits) V.plain_tpr = 0;
     }

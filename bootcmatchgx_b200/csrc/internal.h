@@ -38,6 +38,27 @@ long long launch_count();
 // k-th allocation of that set-up) and disarms it on return. Zero in production.
 extern thread_local long long t_fail_alloc_countdown;
 
+// Builds a form that a hierarchy is faster with and can do without (the stencil form, chain plans): false when
+// the device memory does not suffice, and the caller goes on without it. Its allocations are not
+// counted by BCMGX_TEST_FAIL_ALLOC; BCMGX_TEST_FAIL_FORM=k fails the k-th of every form.
+struct FormAllocScope {
+    const long long outer = t_fail_alloc_countdown;
+    FormAllocScope();
+    ~FormAllocScope() { t_fail_alloc_countdown = outer; }
+};
+template <typename F>
+bool optional_form(F&& build)
+{
+    FormAllocScope scope;
+    try {
+        build();
+        return true;
+    } catch (const Error& e) {
+        if (e.code != BCMGX_ERR_OOM) throw;
+        return false;
+    }
+}
+
 #define BCMGX_CUDA(call)                                                                       \
     do {                                                                                       \
         cudaError_t e_ = (call);                                                               \

@@ -2375,6 +2375,8 @@ void build_stencil(DevCsr& A, bool need64, cudaStream_t s)
     note_launch(); k_pat_rep<<<gs_grid(n), 256, 0, s>>>(n, A.row.p, form.p, rep.p, len.p);
     note_launch(); k_st_forms<<<gs_grid(nform * 32), 256, 0, s>>>(nform, A.row.p, A.col.p, A.val.p, rep.p, len.p, foffs.p, fvals.p);
     BCMGX_CHECK_LAUNCH();
+    ho.release();   // before the values are stored
+    hf.release();
     std::vector<int> ho_offs(nform * 32), ho_len(nform);
     std::vector<double> ho_vals(nform * 32);
     BCMGX_CUDA(cudaMemcpyAsync(ho_offs.data(), foffs.p, sizeof(int) * nform * 32, cudaMemcpyDeviceToHost, s));

@@ -1961,12 +1961,20 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
     int best = default_tpr(n, A.nnz);
     float best_ms = 1e30f;
     // candidates: 1..16 threads per row, the staged kernel with 1, 2, 4 and 8 (coded negative),
-    // and the sliced kernel (its copy of the matrix is built for the trial and kept if it wins)
-    build_sliced(A, s);
-    build_stencil(A, need64, s);
+    // and the sliced and stencil kernels, whose copies of the matrix are built for their trials. The sliced
+    // copy goes before the stencil's comes, so that the trials never hold both (on 7-point 256^3
+    // they would be the peak of the set-up); the caller builds it again when it wins.
+    bool room = true;
     for (int t : {1, 2, 4, 8, 16, -1, -2, -4, -8, kSlicedCode, kStencilCode}) {
-        if (t == kSlicedCode && !A.sl_ptr.p) continue;
-        if (t == kStencilCode && !A.st_form.p) continue;
+        if (t == kSlicedCode) {
+            build_sliced(A, s);
+            if (!A.sl_ptr.p) continue;
+        }
+        if (t == kStencilCode) {
+            release_sliced(A);
+            room = optional_form([&] { build_stencil(A, need64, s); });
+            if (!room || !A.st_form.p) continue;
+        }
         const bool own = t == kSlicedCode || t == kStencilCode;
         const int tp = own ? 1 : t < 0 ? -t : t, stage = t == kStencilCode ? 3 : t == kSlicedCode ? 2 : t < 0 ? 1 : 0;
         auto launch = [&] {
@@ -1989,8 +1997,8 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (best != kSlicedCode) release_sliced(A);
     if (best != kStencilCode) release_stencil(A);
+    if (!room) return best;   // not for good: with more memory the stencil kernels may win
     std::lock_guard<std::mutex> g(g_tune_mu);
     g_tune_cache[key] = best;
     tune_cache_store(key, best);

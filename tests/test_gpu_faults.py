@@ -6,6 +6,9 @@ Every failure is made on the host or by a bounded device wait that runs out on p
 * an injected allocation failure (BCMGX_TEST_FAIL_ALLOC=k fails the k-th device allocation of a
   set-up) makes bcmgx_setup return BCMGX_ERR_OOM at every point of the set-up, and after 100 such
   set-ups the device memory pool holds no more than before;
+* the forms that a hierarchy can do without (the stencil form, chain plans) are left out when their
+  allocations fail (BCMGX_TEST_FAIL_FORM=k fails the k-th of each): the set-up succeeds, and the results are
+  the same, and trying them does not raise the set-up's peak;
 * a suitor step budget of 0 (BCMGX_TEST_SUITOR_BUDGET) makes the matching give up and the set-up
   return BCMGX_ERR_TIMEOUT;
 * the staged row kernels' stage waits (BCMGX_TEST_STAGE_FAULT=<ns> drops block 0's first tile copy
@@ -14,9 +17,15 @@ Every failure is made on the host or by a bounded device wait that runs out on p
   context succeeds.
 The reference has no counterpart: it exits on every error (BCMGX/src/utility/mpi.h:25-32).
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -97,6 +106,68 @@ def test_injected_allocation_failure(bx, cuda, monkeypatch):
     x, info = h.solve(A @ xs)
     assert info["status"] == 0
     h.free()
+
+
+@pytest.mark.parametrize("stored", [False, True])
+def test_forms_are_left_out_without_room(bx, cuda, monkeypatch, stored):
+    import torch
+    row, col, val, A = lap(bx, 7, (24, 23, 22))
+    if stored:   # values of their own everywhere
+        S = sp.diags(np.random.default_rng(3).uniform(0.5, 2.0, A.shape[0]))
+        A = (S @ A @ S).tocsr()
+        row, col, val = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+    b = A @ np.random.default_rng(1).uniform(-1, 1, A.shape[0])
+    monkeypatch.setenv("BCMGX_TPR", "65,2")   # level 0: the stencil kernels where there is the form
+    prm = fcg(bx, rtol=1e-8, vcycle_precision="FP32")
+    outs, forms, launches = [], [], []
+    torch.cuda.synchronize()
+    base = pool_used_bytes()
+    for k in range(16):
+        monkeypatch.setenv("BCMGX_TEST_FAIL_FORM", str(k))
+        h = bx.prec_setup(row, col, val, prm)
+        forms.append(h.info()["index_bytes"][0])
+        c0 = bx.lib().bcmgx_launch_count()
+        outs.append(h.solve(b))
+        launches.append(bx.lib().bcmgx_launch_count() - c0)
+        h.free()
+        torch.cuda.synchronize()
+        assert pool_used_bytes() <= base
+    assert forms[0] == -1 and forms[1] > 0
+    assert launches[1] > launches[0]   # no chain either
+    assert forms[15] == -1 and launches[15] == launches[0]   # fewer allocations than 15: all there again
+    for x, info in outs[1:]:
+        assert info["niter"] == outs[0][1]["niter"] and np.array_equal(x, outs[0][0])
+
+
+PEAK = r"""
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import torch
+import bootcmatchgx_b200 as bx
+from cuda.bindings import driver, runtime as rt
+g = 100
+row, col, val = bx.diffusion_7p(g, g, g, np.exp(np.random.default_rng(1).standard_normal(g ** 3)))
+dev = [torch.from_numpy(a).cuda() for a in (row, col, val)]
+torch.cuda.synchronize()
+_, pool = rt.cudaDeviceGetDefaultMemPool(0)
+high = rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+rt.cudaMemPoolSetAttribute(pool, high, driver.cuuint64_t(0))
+h = bx.prec_setup(*dev, bx.params_default(solver="FCG", preconditioner="BCMG", dispnorm=0))
+print(int(rt.cudaMemPoolGetAttribute(pool, high)[1]))
+"""
+
+
+def test_trials_do_not_raise_the_peak(cuda):
+    """The most memory that a first set-up (which times the row kernels) holds, with the stencil form's trial and
+    without, in a process each. (In FP64, where the form that stays is smaller than what the aggregation holds.)"""
+    peak = []
+    for stencil in ("0", "1"):
+        r = subprocess.run([sys.executable, "-c", PEAK, ROOT], env={**os.environ, "BCMGX_STENCIL": stencil},
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        peak.append(int(r.stdout.split()[-1]))
+    assert peak[1] <= peak[0] * 1.02, peak
 
 
 def test_suitor_budget_exhausted(bx, cuda, monkeypatch):
