@@ -203,8 +203,7 @@ void choose_level_kernels(bcmgx_hierarchy* H, bool chains)
                 V.A.tpr = 1;
                 continue;
             }
-            // a level that has no stencil form (a forced code, or a matrix of the same size as the one
-            // the code was tuned on): the sliced kernels, which take any level; without room for the
+            // a level that has no stencil form (a forced code): the sliced kernels, which take any level; without room for the
             // form the plain ones, which need none and add a row's entries in the same order
             code = room ? kSlicedCode : 1;
         }

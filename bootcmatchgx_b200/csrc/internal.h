@@ -240,6 +240,8 @@ inline int stencil_box(int u, const StencilOffs& so)
 // blocks of 4 offsets that the stencil kernels are compiled for: the least of these with room for u
 inline int stencil_blocks(int u) { return u <= 8 ? 2 : u <= 16 ? 4 : u <= 28 ? 7 : 8; }
 void build_stencil(DevCsr& A, bool need64, cudaStream_t s);
+// Whether a sample of A's rows leaves the form possible (one host round trip where the row lengths do).
+bool stencil_like(const DevCsr& A, cudaStream_t s);
 void release_stencil(DevCsr& A);
 
 // A small level's sweep chains as one cluster launch (chain.cu): ctas blocks of R rows, the level's

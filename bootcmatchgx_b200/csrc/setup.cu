@@ -2318,6 +2318,46 @@ __global__ void k_st_fill(int n, long total, int u, StencilOffs so, const int* _
     }
 }
 
+// like = 1 when 256 rows spread over the matrix, of at most 32 entries each, take their columns from at most
+// 32 offsets, as the rows of a stencil must.
+constexpr int kStProbe = 256;
+__global__ void __launch_bounds__(kStProbe) k_stencil_probe(int n, const int* __restrict__ row, const int* __restrict__ col, int* like)
+{
+    constexpr int kSlots = 1024, kFree = (int)0x80000000;   // no offset of an int32 column
+    __shared__ int keys[kSlots];
+    __shared__ int count;
+    for (int i = threadIdx.x; i < kSlots; i += kStProbe) keys[i] = kFree;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    const int r = (int)((long)threadIdx.x * n / kStProbe);
+    // a thread that sees more than 32 stops, so at most 32 + 256 of the slots are taken
+    for (int j = row[r]; j < row[r + 1] && *(volatile int*)&count <= 32; j++) {
+        const int off = col[j] - r;
+        for (unsigned h = vc_hash((unsigned)off);; h = (h + 1) & (kSlots - 1)) {
+            const int old = atomicCAS(keys + h, kFree, off);
+            if (old == kFree) atomicAdd(&count, 1);
+            if (old == kFree || old == off) break;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *like = count <= 32 ? 1 : 0;
+}
+
+bool stencil_like(const DevCsr& A, cudaStream_t s)
+{
+    const char* env = std::getenv("BCMGX_STENCIL");
+    if ((env && env[0] == '0') || A.n <= 0 || A.max_row <= 0 || A.max_row > 32) return false;
+    DBuf<int> like;
+    like.alloc(1, s);
+    note_launch();
+    k_stencil_probe<<<1, kStProbe, 0, s>>>(A.n, A.row.p, A.col.p, like.p);
+    BCMGX_CHECK_LAUNCH();
+    int h = 0;
+    BCMGX_CUDA(cudaMemcpyAsync(&h, like.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    BCMGX_CUDA(cudaStreamSynchronize(s));
+    return h != 0;
+}
+
 void build_stencil(DevCsr& A, bool need64, cudaStream_t s)
 {
     if (A.st_form.p) return;

@@ -1892,10 +1892,13 @@ void time_block_kernels(bcmgx_hierarchy* H, int K, int reps, double* out)
 // candidate 1..16 of the plain kernel and 1, 2, 4, 8 of the staged one, and the fastest is kept.
 // The result is a code: the threads per row, negative for the staged kernel (the two kernels
 // sum a row in the same order, so that choice does not change results). Codes are cached per
-// (rows, nnz, precision) for the life of the process, so repeated set-ups of same-shaped
+// (rows, nnz, kind) for the life of the process, so repeated set-ups of same-shaped
 // matrices reuse them; when the environment variable BCMGX_TUNE_CACHE names a file, the cache is
 // also read from it at the first use and every new result is appended to it (one "rows nnz
-// precision code" line each).
+// kind code" line each). kind: 1 for an FP32 level, + 2 for a coded one, + 4 for one that looks like a stencil
+// (stencil_like): of two matrices of one size, a box and its rows in another order, the first may be
+// for the stencil kernels and the second has no such form.
+constexpr int kKindStencil = 4;
 static std::mutex g_tune_mu;
 static std::map<std::tuple<int, int64_t, int>, int> g_tune_cache;
 static bool g_tune_loaded = false;
@@ -1909,11 +1912,11 @@ static void tune_cache_load()
     FILE* f = std::fopen(path, "r");
     if (!f) return;
     long long z;
-    int n, prec, t;
-    while (std::fscanf(f, "%d %lld %d %d", &n, &z, &prec, &t) == 4)
+    int n, kind, t;
+    while (std::fscanf(f, "%d %lld %d %d", &n, &z, &kind, &t) == 4)
         if (t == 1 || t == 2 || t == 4 || t == 8 || t == 16 || t == 32 || t == -1 || t == -2 || t == -4 || t == -8 ||
-            t == kSlicedCode || t == kStencilCode)
-            g_tune_cache[std::make_tuple(n, (int64_t)z, prec)] = t;
+            t == kSlicedCode || (t == kStencilCode && (kind & kKindStencil)))
+            g_tune_cache[std::make_tuple(n, (int64_t)z, kind)] = t;
     std::fclose(f);
 }
 
@@ -1932,14 +1935,27 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
     DevCsr& A = V.A;
     const int n = A.n;
     if (n < kTuneMinRows) return default_tpr(n, A.nnz);
-    // coded levels are tuned apart: a matrix of the same size with other values has other kernels
-    const auto key = std::make_tuple(n, A.nnz, (f32 ? 1 : 0) | (A.vcode.p ? 2 : 0));
+    int kind = (f32 ? 1 : 0) | (A.vcode.p ? 2 : 0);
+    int box = 0, other = 0;   // the codes of the size's stencils and of its other matrices, 0: not timed yet
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         tune_cache_load();
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) return it->second;
+        auto cached = [&](int k) {
+            auto it = g_tune_cache.find(std::make_tuple(n, A.nnz, k));
+            return it == g_tune_cache.end() ? 0 : it->second;
+        };
+        box = cached(kind | kKindStencil);
+        other = cached(kind);
     }
+    // (where only stencils of the size are known, for the stencil kernels, building the form tells by itself)
+    bool like = (box == kStencilCode && !other) || stencil_like(A, s);
+    if (like && box == kStencilCode) {
+        const bool room = optional_form([&] { build_stencil(A, need64, s); });
+        if (!room || A.st_form.p) return box;
+        like = false;   // the sampled rows look like a stencil's, the others do not
+    }
+    if (like ? box : other) return like ? box : other;
+    if (like) kind |= kKindStencil;
     DBuf<double> a, b, c;
     DBuf<float> a32, b32, c32;
     if (f32) {
@@ -1971,6 +1987,7 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
             if (!A.sl_ptr.p) continue;
         }
         if (t == kStencilCode) {
+            if (!like) continue;
             release_sliced(A);
             room = optional_form([&] { build_stencil(A, need64, s); });
             if (!room || !A.st_form.p) continue;
@@ -1997,9 +2014,11 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (best != kSlicedCode) release_sliced(A);
     if (best != kStencilCode) release_stencil(A);
     if (!room) return best;   // not for good: with more memory the stencil kernels may win
     std::lock_guard<std::mutex> g(g_tune_mu);
+    const auto key = std::make_tuple(n, A.nnz, kind);
     g_tune_cache[key] = best;
     tune_cache_store(key, best);
     return best;
