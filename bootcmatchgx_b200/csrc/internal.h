@@ -208,6 +208,7 @@ struct DevCsr {
     StencilOffs st_offs {};
     int st_u = 0, st_nform = 0;
     int st_box = 0;   // line length of a 27-point box (stencil_box), 0: another stencil
+    int st_rows = 0;  // rows per lane of the box kernel (1, 2 or 4) that BCMGX_BOX_ROWS forces, 0: launch_box's rule
     DBuf<unsigned char> st_form;
     DBuf<unsigned> st_mask;
     DBuf<double> st_tab64, st_val64;
@@ -226,7 +227,7 @@ void release_sliced(DevCsr& A);
 // Stencil form of a square level whose rows take their columns from at most 32 offsets and at most
 // 255 forms (three host round trips); leaves A.st_form empty when the level does not qualify.
 // need64: the FP64 values are wanted too (always when the level has no FP32 ones). BCMGX_STENCIL=0
-// turns it off.
+// turns it off; BCMGX_BOX_ROWS=1, 2 or 4 fixes the rows per lane on 27-point boxes.
 constexpr int kStencilCode = 65;
 // Line length s of the 27 offsets pl[a] + (b - 1) s + (c - 1) of a box (three planes, pl[1] = 0), else 0.
 inline int stencil_box(int u, const StencilOffs& so)

@@ -2478,6 +2478,9 @@ void build_stencil(DevCsr& A, bool need64, cudaStream_t s)
     A.st_u = u;
     A.st_nform = nform;
     A.st_box = stencil_box(u, so);
+    const char* rows = std::getenv("BCMGX_BOX_ROWS");
+    const int forced = rows ? std::atoi(rows) : 0;
+    A.st_rows = forced == 1 || forced == 2 || forced == 4 ? forced : 0;
 }
 
 void finish_level_matrix(Level& V, bool want_f32, cudaStream_t s)

@@ -335,43 +335,54 @@ static void launch_sliced(const DevCsr& A, SlSrc<VS> sv, const XT* x, const FT* 
     BCMGX_CHECK_LAUNCH();
 }
 
-// Rows per lane of the 27-point box kernel on a level (1: the general stencil kernel). More rows a
-// lane load less of x, but leave fewer warps: measured with 1 / 2 / 4 rows, FP32 sweeps take 47.6 / 28.5
-// / 26.8 us at 4.1 M rows, 12.2 / 9.7 / 10.1 at 1 M, 6.4 / 4.4 / 5.3 at 262 k, 3.9 / 3.6 / 4.2 at 125 k;
-// FP32 residuals 44.2 / 28.7 / 22.2, 11.3 / 9.0 / 8.6, 5.8 / 4.8 / 4.1, 3.9 / 3.4 / 3.6; FP64 sweeps 16.0 /
-// 15.1 / 16.5 at 1 M (the product and dots 79.0 / 62.1 / 64.3 at 4.1 M), 15.6 / 14.5 / 12.9 at 886 k, 6.6 /
-// 7.3 / 6.1 at 262 k, 4.3 / 5.4 / 5.1 at 125 k.
-static int box_rows(const DevCsr& A, int op, size_t xbytes)
+// Rows per lane of the 27-point box kernel on a level (1: the general stencil kernel). More rows a lane load
+// less of x and keep fewer blocks on an SM (FP32 sweeps 4 with two rows and 3 with four, FP64 sweeps and
+// residuals 3 and 2). The grid is what is resident, and all of its lanes work for as many rounds as
+// the fullest: a sweep takes about 2.3 us and its rounds, one of four rows costing as much as 1.375 (FP32)
+// or 1.3 (FP64) of two rows. So the fewer rounds by that measure decide, not the rows alone. us with 1 / 2 / 4 rows
+// (rounds of 2 / 4; the choice is at most 4 % off the best at the 17 boxes measured): FP32 262 k rows 6.4 / 4.5 / 5.2 (1 / 1), 394 k 6.6 / 6.0 / 5.3 (2 / 1), 512 k 8.4 / 6.6 / 7.6
+// (2 / 2), 1.0 M 12.2 / 9.5 / 9.9 (4 / 3), 1.7 M 19.2 / 15.0 / 14.0 (6 / 4), 4.1 M 47.9 / 28.9 / 26.9 (14 / 10); FP64
+// 262 k 6.6 / 7.4 / 6.1 (2 / 1), 394 k 8.4 / 7.8 / 9.5 (2 / 2), 512 k 10.5 / 10.5 / 9.7 (3 / 2), 886 k 15.0 / 13.8 / 12.2
+// (4 / 3), 1.0 M 16.1 / 15.0 / 16.2 (5 / 4), 2.0 M 28.9 / 24.4 / 23.5 (9 / 7), 4.1 M 58.5 / 50.3 / 47.4 (19 / 14). Below
+// 200 k rows all three are within 0.3 us (FP32 152 k 3.9 / 4.2 / 4.1) and one row needs no box.
+// FP32 residuals, with 5 and 4 blocks, are best with four rows (262 k 5.8 / 4.7 / 4.0, 1.0 M 11.3 / 9.1 / 8.6, 4.1 M 44.1 /
+// 28.6 / 22.2; only 697 k is 5 % better with two). In the FP64 product the rounds are the same with both; with its
+// dots, four rows take 13.2 against 14.2 us at 262 k, 22.8 / 24.6 at 1.0 M, 37.5 / 39.0 at 2.6 M, and 64.7 / 61.9 at 4.1 M.
+constexpr int kBoxMinRows = 200000, kBoxProductRows = 3000000;
+
+template <int OP, typename VT, typename XT, typename FT, typename MT, typename YT>
+static bool launch_box(const DevCsr& A, const VT* vals, const XT* x, const FT* f, const MT* M, YT* y, double alpha,
+    double beta, const int* skip, cudaStream_t s)
 {
-    if (A.st_box <= 0 || A.n < 200000) return 1;
-    if (xbytes == 8) return A.n < 950000 ? 4 : 2;
-    return op == OP_RESID || A.n >= 2000000 ? 4 : 2;
+    if (A.st_box <= 0 || A.st_rows == 1 || (!A.st_rows && A.n < kBoxMinRows)) return false;
+    const int bs = A.st_box;
+    const size_t smem = (size_t)A.st_nform * 36 * sizeof(VT);
+    auto k2 = k_rowop_box27<OP, 2, VT, XT, FT, MT, YT>;
+    auto k4 = k_rowop_box27<OP, 4, VT, XT, FT, MT, YT>;
+    auto resident = [&](auto kern) {
+        ensure_smem_limit((const void*)kern, smem);
+        return (long)blocks_per_sm((const void*)kern, kStThreads, smem) * num_sms();
+    };
+    auto blocks = [&](int P) { return (long)ceil_div(((long)A.n + (long)P * bs - 1) / ((long)P * bs) * bs, kStThreads); };
+    const long r2 = resident(k2), r4 = resident(k4), b2 = blocks(2), b4 = blocks(4);
+    bool four;
+    if (A.st_rows) four = A.st_rows == 4;
+    else if (OP == OP_AXPBY) four = A.n < kBoxProductRows;
+    else if (OP == OP_RESID && sizeof(XT) == 4) four = true;
+    else four = ceil_div(b4, r4) * (sizeof(XT) == 4 ? 1.375 : 1.3) < (double)ceil_div(b2, r2);
+    launch_dep<0>(four ? k4 : k2, (int)std::max<long>(1, four ? std::min(b4, r4) : std::min(b2, r2)), kStThreads, smem, s, A.n, bs,
+        A.st_offs.o[4], A.st_offs.o[22], (const unsigned char*)A.st_form.p, (const unsigned*)A.st_mask.p, A.st_nform, vals,
+        x, f, M, y, alpha, beta, skip);
+    BCMGX_CHECK_LAUNCH();
+    return true;
 }
 
 template <int OP, bool TAB, typename VT, typename XT, typename FT, typename MT, typename YT>
 static void launch_stencil(const DevCsr& A, const VT* vals, const XT* x, const FT* f, const MT* M, YT* y, double alpha,
     double beta, const int* skip, cudaStream_t s)
 {
-    if constexpr (TAB) {
-        const int P = box_rows(A, OP, sizeof(XT));
-        if (P > 1) {
-            const int bs = A.st_box;
-            const size_t smem = (size_t)A.st_nform * 36 * sizeof(VT);
-            const long items = ((long)A.n + (long)P * bs - 1) / ((long)P * bs) * bs;
-            auto go = [&](auto kern) {
-                ensure_smem_limit((const void*)kern, smem);
-                const int per_sm = blocks_per_sm((const void*)kern, kStThreads, smem);
-                const int grid = (int)std::max<long>(1, std::min<long>(ceil_div(items, kStThreads), (long)per_sm * num_sms()));
-                launch_dep<0>(kern, grid, kStThreads, smem, s, A.n, bs, A.st_offs.o[4], A.st_offs.o[22],
-                    (const unsigned char*)A.st_form.p, (const unsigned*)A.st_mask.p, A.st_nform, vals, x, f, M, y, alpha,
-                    beta, skip);
-                BCMGX_CHECK_LAUNCH();
-            };
-            if (P == 4) go(k_rowop_box27<OP, 4, VT, XT, FT, MT, YT>);
-            else go(k_rowop_box27<OP, 2, VT, XT, FT, MT, YT>);
-            return;
-        }
-    }
+    if constexpr (TAB)
+        if (launch_box<OP>(A, vals, x, f, M, y, alpha, beta, skip, s)) return;
     const int nb = stencil_blocks(A.st_u);
     const size_t smem = TAB ? (size_t)A.st_nform * 4 * nb * sizeof(VT) : 0;
     auto go = [&](auto kern) {

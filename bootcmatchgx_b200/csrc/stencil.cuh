@@ -40,8 +40,8 @@ extern __shared__ __align__(128) unsigned char st_smem[];
 // y = alpha A x + beta y, y = f - A x, or one l1-Jacobi sweep (the operations of k_rowop). With stored
 // values HBM bounds it: one FP32 sweep of the 7-point 256^3 diffusion level streams 755 MB instead of
 // 1.27 GB and takes 142 us (5.3 TB/s) instead of 224 with int32 columns. With the table the loads of x
-// do: 7-point 100^3 7.0 us instead of 10.6 with pattern-indexed slices, 27-point 160^3 48.6 instead of
-// 70.6 (k_rowop_box27 below: 27.5). u: the offsets of the stencil, stencil_blocks(u) == NB. TAB: vals is the table of the forms' values (nform
+// do: 7-point 100^3 7.0 us instead of 10.6 with pattern-indexed slices, 27-point 160^3 47.9 instead of
+// 70.6 (k_rowop_box27 below: 26.9). u: the offsets of the stencil, stencil_blocks(u) == NB. TAB: vals is the table of the forms' values (nform
 // rows of 4 NB, dynamic shared memory holds it); else the stored values.
 template <int OP, int NB, bool TAB, typename T, typename XT, typename FT, typename MT, typename YT>
 __global__ void __launch_bounds__(kStThreads) k_rowop_stencil(int n, int u, StencilOffs so,
@@ -135,9 +135,9 @@ __global__ void __launch_bounds__(kStThreads) k_rowop_stencil(int n, int u, Sten
 // all of one form with every offset (the inside of the box) takes the values as broadcasts and tests
 // nothing; in any other, a value is loaded when one of the P rows has its column and added to the
 // rows that have it. Rows q P s + p s + t (t < s, p < P) of a lane: the last group may pass n.
-// Measured at 160^3 (FP32 sweep): k_rowop_stencil 48.6 us (240 warp instructions per 32 rows), P = 2
-// 29.5, P = 4 27.5 us: 2.5 TB/s on its 69 MB of vectors and form bytes, most of them in L2, bound by the
-// loads of x and by issue. An FP64 product and its dots 96.6 -> 63.8 us.
+// Measured at 160^3 (FP32 sweep): k_rowop_stencil 47.9 us (240 warp instructions per 32 rows), P = 2
+// 28.9, P = 4 26.9 us: 2.6 TB/s on its 70 MB of vectors and form bytes, most of them in L2, bound by the
+// loads of x and by issue. An FP64 product and its dots 78.7 -> 61.9 us (P = 2). launch_box chooses P.
 template <int OP, int P, typename T, typename XT, typename FT, typename MT, typename YT>
 __global__ void __launch_bounds__(kStThreads) k_rowop_box27(int n, int s, int pl0, int pl2,
     const unsigned char* __restrict__ form, const unsigned* __restrict__ fmask, int nform, const T* __restrict__ vals,

@@ -38,9 +38,10 @@ def banded(n, offs, seed):
     return (B + sp.diags(d)).tocsr()
 
 
-# (matrix, does level 0 have the form): table and stored values; 7 and 27 offsets and the least and most of every
-# compiled width (1, 8, 9, 16, 17, 28, 29, 32 offsets are 2 m + 1 or one-sided counts: m = 4 -> 9, 8 -> 17, 14 -> 29,
-# 15 -> 31); sizes that leave a ragged last slice and block; a matrix smaller than one slice; a matrix without the form
+# (matrix, does level 0 have the form): table and stored values; 7 and 27 offsets and symmetric bands of 3, 9, 15, 17,
+# 29 and 31, the least and most odd counts of the compiled widths (8, 16, 28 and 32 offsets: a symmetric matrix with a
+# diagonal has an odd number); sizes that leave a ragged last slice and block; a matrix smaller than one slice; a matrix
+# without the form
 CASES = {
     "lap27": (lambda bx: matrix(bx, ("lap27", (37, 29, 23))), True),
     "lap7": (lambda bx: matrix(bx, ("lap7", (33, 31, 25))), True),
@@ -49,6 +50,7 @@ CASES = {
     "band9": (lambda bx: banded(3001, (1, 2, 40, 200), None), True),
     "band9_stored": (lambda bx: banded(4003, (1, 2, 40, 200), 4), True),
     "band3_stored": (lambda bx: banded(999, (1,), 5), True),
+    "band15": (lambda bx: banded(3100, (1, 2, 3, 5, 7, 11, 13), None), True),
     "band17": (lambda bx: banded(2050, (1, 2, 3, 5, 7, 11, 13, 17), None), True),
     "band29_stored": (lambda bx: banded(9000, tuple(range(1, 15)), 6), True),
     "band31": (lambda bx: banded(2500, tuple(range(1, 16)), None), True),
@@ -73,9 +75,37 @@ def test_stencil_solve_bit_identical(bx, cuda, monkeypatch, name, prec):
     assert np.array_equal(x0, x1)
 
 
-def test_stencil_reads_only_a_rows_own_entries(bx, cuda, monkeypatch):
+def solve_both(bx, monkeypatch, A, kw):
+    b = A @ np.random.default_rng(3).uniform(-1, 1, A.shape[0])
+    x0, i0, _ = setup_solve(bx, monkeypatch, A, b, 1, **kw)
+    x1, i1, h1 = setup_solve(bx, monkeypatch, A, b, STENCIL, **kw)
+    assert h1["index_bytes"][0] == -1
+    assert i0["niter"] == i1["niter"] and np.array_equal(x0, x1)
+
+
+# the box kernel with every number of rows a lane: lines whose number is not a multiple of 2 or of 4 (the last group
+# passes the end), lines shorter and longer than a warp, planes of one line less than a group, and a single group
+@pytest.mark.parametrize("prec", ["FP64", "FP32"])
+@pytest.mark.parametrize("rows", [1, 2, 4])
+@pytest.mark.parametrize("grid", [(37, 29, 23), (31, 6, 11), (70, 3, 7), (3, 5, 41), (33, 4, 4)])
+def test_box_rows_bit_identical(bx, cuda, monkeypatch, grid, rows, prec):
+    monkeypatch.setenv("BCMGX_BOX_ROWS", str(rows))
+    solve_both(bx, monkeypatch, matrix(bx, ("lap27", grid)), dict(vcycle_precision=prec, rtol=1e-8))
+
+
+# the sizes where the rule takes other rows: two and four for the FP32 and FP64 sweeps (64x61x67: 2 and 4, 73x75x72: 4 and
+# 2), and two for the product above 3 M rows
+@pytest.mark.parametrize("grid,prec", [((64, 61, 67), "FP32"), ((64, 61, 67), "FP64"), ((73, 75, 72), "FP32"),
+                                       ((73, 75, 72), "FP64"), ((163, 151, 123), "FP32")])
+def test_box_rule_bit_identical(bx, cuda, monkeypatch, grid, prec):
+    solve_both(bx, monkeypatch, matrix(bx, ("lap27", grid)), dict(vcycle_precision=prec, rtol=1e-6))
+
+
+@pytest.mark.parametrize("rows", [0, 2, 4])
+def test_stencil_reads_only_a_rows_own_entries(bx, cuda, monkeypatch, rows):
     """One sweep of the preconditioner on a vector with an Inf: the rows that have no entry in its column keep the
-    plain kernel's bits (an offset that a row lacks must not bring Inf * 0 into its sum)."""
+    plain kernel's bits (an offset that a row lacks must not bring Inf * 0 into its sum). rows: a lane's in the box
+    kernel; 0: the general stencil kernel, which takes a box of this size."""
     import torch
     A = matrix(bx, ("lap27", (21, 19, 17)))
     n = A.shape[0]
@@ -83,6 +113,7 @@ def test_stencil_reads_only_a_rows_own_entries(bx, cuda, monkeypatch):
     r[n // 2 + 3] = np.inf
     r[20] = np.nan      # the end of an x line: row 21 starts the next one and has no entry there
     t = torch.from_numpy(r).to(cuda)
+    monkeypatch.setenv("BCMGX_BOX_ROWS", str(rows))
     outs = []
     for code in (1, STENCIL):
         monkeypatch.setenv("BCMGX_TPR", str(code))
@@ -112,7 +143,7 @@ def test_stencil_code_on_another_matrix(bx, cuda, monkeypatch):
 @pytest.mark.parametrize("prec", ["FP64", "FP32"])
 @pytest.mark.parametrize("grid,k", [((40, 37, 33), 32), ((41, 35, 39), 19), ((70, 61, 66), 4), ((71, 67, 59), 3), ((113, 101, 97), 1)])
 def test_stencil_block_solve(bx, cuda, monkeypatch, grid, k, prec):
-    """Block solves on a 27-point box (blk_box_rows: four rows of a slot share their gathers), with ragged lines,
+    """Block solves on a 27-point box (blk_box_rows: two or four rows of a slot share their gathers), with ragged lines,
     planes that are not a multiple of four lines and 1 to 32 columns, against the CSR block kernels. The sweeps
     add the same terms in the same order; the dot products' partial sums do not, so the solutions agree to
     the rounding of those sums (1e-16 each, carried through some 30 iterations)."""
