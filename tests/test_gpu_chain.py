@@ -24,7 +24,8 @@ def multi_launch_cycle(monkeypatch):
 
 
 def cycle_and_solve(bx, monkeypatch, A, chain, S=2, **kw):
-    """One cycle and one solve with S threads per row on every level."""
+    """One cycle and two solves with S threads per row on every level: the first starts on the stream, the second
+    is the captured one (use_graph = 1)."""
     import torch
     monkeypatch.setenv("BCMGX_CHAIN", chain)
     monkeypatch.setenv("BCMGX_TPR", str(S))
@@ -37,7 +38,12 @@ def cycle_and_solve(bx, monkeypatch, A, chain, S=2, **kw):
     v = h.prec_apply(torch.from_numpy(r).cuda()).cpu().numpy()
     launches = bx.lib().bcmgx_launch_count() - c0
     # (one row: the start-up step is exact and leaves a zero residual, which the iteration refuses)
-    x, info = h.solve(A @ rng.uniform(-1, 1, n)) if n > 1 else (v, {"niter": 1})
+    x, info = v, {"niter": 1}
+    if n > 1:
+        b = A @ rng.uniform(-1, 1, n)
+        x, info = h.solve(b)
+        x2, info2 = h.solve(b)
+        assert info2["niter"] == info["niter"] and np.array_equal(x, x2)
     h.free()
     return v, x, info, launches
 
@@ -74,7 +80,7 @@ def test_chain_bit_identical(bx, cuda, monkeypatch, name, S, prec):
                                 dict(prerelax_sweeps=1, postrelax_sweeps=2), dict(prerelax_sweeps=0, postrelax_sweeps=3),
                                 dict(use_graph=0)])
 def test_chain_cycles(bx, cuda, monkeypatch, kw):
-    """Second visits of a level (a chain from its iterate), chains of 1 to 3 sweeps, the stream driver."""
+    """Second visits of a level (a chain from its iterate), chains of 1 to 3 sweeps, the stream driver alone."""
     A = matrix(bx, ("lap7", (40, 37, 33)))
     v0, x0, i0, _ = cycle_and_solve(bx, monkeypatch, A, "0", **kw)
     v1, x1, i1, _ = cycle_and_solve(bx, monkeypatch, A, "1", **kw)
