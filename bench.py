@@ -316,33 +316,37 @@ def time_vcycle(h, r, stream, reps=10):
     return e0.elapsed_time(e1) / reps
 
 
+def matrix_bytes(n, nnz, index_bytes, coded, value_bytes):
+    """Bytes of a level's matrix that one pass of its row kernel streams. index_bytes as the hierarchy reports them: 4 or
+    2 per entry beside its value (1 byte when the level is coded) and the row offsets; 0, pattern-indexed
+    rows, one byte per row in their place; -1, the stencil form: one byte per row and, unless a table holds the
+    values (coded), a stored value for every row and offset of the stencil (as many offsets as the longest rows have
+    entries, here the entries per row rounded up), no row offsets."""
+    if index_bytes < 0:
+        return n + (0 if coded else -(-nnz // n) * n * value_bytes)
+    return (index_bytes + (1 if coded else value_bytes)) * nnz + (n if index_bytes == 0 else 0) + 4 * (n + 1)
+
+
 def vcycle_bytes(inf, pre, post, coarse):
     """Algorithmic bytes of one FP32 V-cycle as the kernels run it: on every level but the last,
     pre + post - 1 l1-Jacobi sweeps over the FP32 matrix (the first pre-sweep starts from zero and
     reads no matrix), the residual, the restriction R r (one entry per fine row) and the
     prolongation x += p x_c[agg]; the coarsest level runs `coarse` FP64 sweeps (the first from
-    zero). Matrix entries
-    count index_bytes + value bytes (1 where the level streams 1-byte value codes, else 4; 8 for the
-    coarsest level's FP64 values; index_bytes 0, pattern-indexed rows, streams 1 byte per row instead; -1, the
-    stencil form, also takes the values from a table where the level has value codes),
-    vectors 4 bytes (8 on the coarsest level); level 0 also reads the FP64 residual and writes the FP64
-    output."""
-    n, z, ib = inf["n"], inf["nnz"], [max(b, 0) for b in inf["index_bytes"]]
-    vb = [(0 if b < 0 else 1) if c else 4 for b, c in zip(inf["index_bytes"], inf["value_codes"])]
+    zero). The matrix counts as matrix_bytes says (FP32 values, FP64 on the coarsest level), vectors 4 bytes (8 on
+    the coarsest level); level 0 also reads the FP64 residual and writes the FP64 output."""
+    n, z, ib, codes = inf["n"], inf["nnz"], inf["index_bytes"], inf["value_codes"]
     total = 0
     for l in range(len(n) - 1):
         nl, zl, nc = n[l], z[l], n[l + 1]
-        mat = (ib[l] + vb[l]) * zl + (nl if ib[l] == 0 else 0)
-        sweep = mat + 4 * (nl + 1) + 16 * nl
-        total += (pre + post - 1) * sweep + 12 * nl
-        total += mat + 4 * (nl + 1) + 12 * nl
+        mat = matrix_bytes(nl, zl, ib[l], codes[l], 4)
+        total += (pre + post - 1) * (mat + 16 * nl) + 12 * nl
+        total += mat + 12 * nl
         total += 4 * (nc + 1) + 8 * nl + 4 * nl + 4 * nc
         total += 8 * nl + 4 * nc + 8 * nl
         if l == 0:
             total += 8 * nl + 4 * nl
     nL, zL = n[-1], z[-1]
-    total += (coarse - 1) * ((ib[-1] + (1 if inf["value_codes"][-1] else 8)) * zL + (nL if ib[-1] == 0 else 0)
-                             + 4 * (nL + 1) + 32 * nL) + 24 * nL
+    total += (coarse - 1) * (matrix_bytes(nL, zL, ib[-1], codes[-1], 8) + 32 * nL) + 24 * nL
     return int(total)
 
 
@@ -447,21 +451,18 @@ def run_ours(a, wl, rank, world, local_rank):
     h32.free()
     h64.free()
     peak, peak_kind = read_peaks()
-    # algorithmic bytes of the format the kernels stream: int16 column offsets (2 B) where the
-    # level has them, else int32 (4 B), or with pattern-indexed rows (index bytes 0) one byte per
-    # row naming its offsets; 1-byte value codes where the level has them, else the 4- or 8-byte
-    # values; bcmgx_spmv on raw CSR arrays always streams int32 + FP64
+    # algorithmic bytes of the format the kernels stream (matrix_bytes); bcmgx_spmv on raw CSR arrays always
+    # streams int32 + FP64
     ib32, ib64 = inf32["index_bytes"][0], inf64["index_bytes"][0]
-    # (the stencil form, index bytes -1: one byte per row, which also names the values of a level with
-    # value codes)
     sten32, sten64 = ib32 < 0, ib64 < 0
-    ib32, ib64 = max(ib32, 0), max(ib64, 0)
+    mat32 = matrix_bytes(n, nnz, ib32, inf32["value_codes"][0], 4)
+    mat64 = matrix_bytes(n, nnz, ib64, inf64["value_codes"][0], 8)
+    ib32 = max(ib32, 0)
     vb32 = (0 if sten32 else 1) if inf32["value_codes"][0] else 4
     vb64 = (0 if sten64 else 1) if inf64["value_codes"][0] else 8
-    rb32, rb64 = (n if ib32 == 0 else 0), (n if ib64 == 0 else 0)
     bytes_spmv = 12 * nnz + 4 * (n + 1) + 16 * n
-    bytes_jac32 = (ib32 + vb32) * nnz + rb32 + 4 * (n + 1) + 16 * n
-    bytes_jac64 = (ib64 + vb64) * nnz + rb64 + 4 * (n + 1) + 32 * n
+    bytes_jac32 = mat32 + 16 * n
+    bytes_jac64 = mat64 + 32 * n
     bytes_jac32_csr = 8 * nnz + 4 * (n + 1) + 16 * n   # the same sweep on int32 columns + FP32 values
     gbs_spmv = bytes_spmv / (spmv_ms * 1e-3) / 1e9
     gbs_jac32 = bytes_jac32 / (k32["jacobi"] * 1e-3) / 1e9
@@ -537,7 +538,7 @@ def run_ours(a, wl, rank, world, local_rank):
                            "fp32_residual_ms": k32["residual"], "fp64_jacobi_ms": k64f["jacobi"],
                            "fp64_jacobi_gbs": gbs_jac64, "fcg_spmv_dots_ms": k64f["fcg_spmv_dots"],
                            # pw = A pv (row kernel) then the three dots (r, pw, oq against pv)
-                           "fcg_spmv_dots_gbs": ((ib64 + vb64) * nnz + rb64 + 4 * (n + 1) + 48 * n) / (k64f["fcg_spmv_dots"] * 1e-3) / 1e9,
+                           "fcg_spmv_dots_gbs": (mat64 + 48 * n) / (k64f["fcg_spmv_dots"] * 1e-3) / 1e9,
                            "fp32_jacobi_fp64_out_ms": k32["jacobi_fp64_out"],
                            "fcg_update_ms": k32["fcg_update"],
                            "fcg_update_gbs": 80 * n / (k32["fcg_update"] * 1e-3) / 1e9},
@@ -549,7 +550,8 @@ def run_ours(a, wl, rank, world, local_rank):
                      "format": ("stencil form (1 byte per row)" if sten32 else
                                 "pattern-indexed rows (1 byte per row)" if ib32 == 0 else f"int{8 * ib32} columns")
                                + ", " + {0: "values from a table", 1: "1-byte value codes"}.get(vb32, "FP32 values"),
-                     "bound": "hbm", "achieved": gbs_jac32, "peak": peak, "unit": "GB/s",
+                     # (the stencil kernels' vectors stay mostly in L2: no DRAM traffic is given for them)
+                     "bound": "loads of x" if sten32 and inf32["value_codes"][0] else "hbm", "achieved": gbs_jac32, "peak": peak, "unit": "GB/s",
                      "frac": gbs_jac32 / peak, "peak_kind": f"{peak_kind} hbm_gbs (copy)",
                      "bytes_per_launch": bytes_jac32,
                      "traffic": (int(TRAFFIC_RATIO[(ib32, vb32, form0)] * bytes_jac32)

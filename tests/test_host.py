@@ -317,3 +317,19 @@ def test_reference_arm_builds_the_same_problems(bx):
         r1, c1, v1 = bx.laplacian_3d(st, 6, 5, 4)
         r2, c2, v2 = O.Matrix.lap3d(st, 6, 5, 4).csr()
         assert np.array_equal(r1, r2) and np.array_equal(c1, c2) and np.array_equal(v1, v2)
+
+
+def test_bench_counts_streamed_bytes():
+    """bench.py's bytes of a pass by the level's format: a stencil level reads no row offsets, with a table of
+    values one byte a row, without one a value for every row and offset of the stencil."""
+    import bench
+    n, z = 1000, 6400   # a 7-point box of 10^3
+    assert bench.matrix_bytes(n, z, 4, 0, 4) == 8 * z + 4 * (n + 1)
+    assert bench.matrix_bytes(n, z, 2, 3, 4) == 3 * z + 4 * (n + 1)
+    assert bench.matrix_bytes(n, z, 0, 3, 4) == z + n + 4 * (n + 1)
+    assert bench.matrix_bytes(n, z, -1, 3, 4) == n
+    assert bench.matrix_bytes(n, z, -1, 0, 4) == n + 7 * n * 4
+    inf = {"n": [n, 100], "nnz": [z, 700], "index_bytes": [4, 2], "value_codes": [2, 0]}
+    csr = bench.vcycle_bytes(inf, 4, 4, 20)
+    stencil = bench.vcycle_bytes(dict(inf, index_bytes=[-1, 2]), 4, 4, 20)
+    assert csr - stencil == 8 * (5 * z + 4 * (n + 1) - n)   # seven sweeps and the residual
