@@ -491,6 +491,8 @@ int bcmgx_batch_get_hierarchy(bcmgx_batch* B, int k, bcmgx_hierarchy** h)
         std::lock_guard<std::mutex> g(mu);
         DeviceScope ds(B->device);
         plan_chains(B->hs[k]);   // the caller may solve with it alone
+        // the chain kernel reads its plan before its dependency wait: the plan is complete when this returns
+        BCMGX_CUDA(cudaStreamSynchronize(B->hs[k]->stream));
         *h = B->hs[k];
     });
 }
