@@ -219,17 +219,20 @@ void scan_exclusive_dev(const int* in, int* out, long n, cudaStream_t s)
 // A block takes 256 consecutive rows: their columns, one contiguous range, go to shared memory with
 // asynchronous copies that are all in flight at once (16 bytes each where the array allows it, 4 at its
 // end), then every lane walks its own row there, 4 words in 128 skipped so that rows of 32 entries do not
-// all meet in one bank. The pass is then bound by
-// the column stream: on the 27-point 160^3 matrix (437 MB of columns) the checked product takes 385 us
-// (415 with 4-byte copies) instead of 910, 236 of them the product, where a warp per row took 655 us for the checks. Rows whose block holds more
-// than kValCap entries, or an offset out of order, are walked by a warp each from global memory.
+// all meet in one bank. The pass is then bound by the column stream: on the 27-point 160^3 matrix (437 MB of
+// columns) the checked product takes 385 us (415 with 4-byte copies) instead of 910, 236 of them the product,
+// where a warp per row took 655 us for the checks. Rows whose block holds more than kValCap entries, or an offset
+// out of order, are walked by a warp each from global memory. A matrix whose rows are that long throughout
+// takes fewer rows a block (R, down to one a warp) while its blocks do not fill the GPU: 5,000 rows of 2,000
+// entries are 20 blocks of 256 rows (their checked product 324 us, with a row a warp 66; 20,000 rows of 1,000
+// entries 249 and 102).
 constexpr int kValRows = 256;
 constexpr int kValCap = 8192;
 
 __device__ __forceinline__ int val_slot(int j) { return j + ((j >> 7) << 2); }   // keeps 16-byte chunks whole
 
 template <bool OFFS>
-__global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long nnz, const int* __restrict__ row,
+__global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long nnz, int R, const int* __restrict__ row,
     const int* __restrict__ col, int* err, int* max_row, int* max_off, short* __restrict__ dcol, int need_diag,
     int* __restrict__ dpos)
 {
@@ -238,9 +241,9 @@ __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long n
     const int tid = threadIdx.x, lane = tid & 31;
     const bool wide = ((size_t)col & 15) == 0;
     int mx = 0, mo = 0, bad = 0;
-    const long ntiles = ((long)n + kValRows - 1) / kValRows;
+    const long ntiles = ((long)n + R - 1) / R;
     for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int r0 = (int)(t * kValRows), nr = min(kValRows, n - r0), r = r0 + tid;
+        const int r0 = (int)(t * R), nr = min(R, n - r0), r = r0 + tid;
         __syncthreads();   // the tile before this one has been read
         for (int i = tid; i <= nr; i += kValRows) rows_s[i] = __ldg(row + r0 + i);
         __syncthreads();
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long n
         const bool all_ok = __syncthreads_and(ok);
         const int b0 = rows_s[0], a0 = wide ? b0 & 3 : 0;   // cols_s starts at entry b0 - a0
         const long total = all_ok ? (long)rows_s[nr] - b0 : 0;   // the rows' ranges follow one another
-        if (all_ok && total <= kValCap) {
+        if (all_ok && R == kValRows && total <= kValCap) {
             const int* src = col + (b0 - a0);
             const int cnt = (int)total + a0, whole = wide ? cnt & ~3 : 0;
             for (int j = 4 * tid; j < whole; j += 4 * kValRows)
@@ -321,6 +324,21 @@ __global__ void __launch_bounds__(kValRows) k_validate(int n, int m, long long n
         if (mx > 0) atomicMax(max_row, mx);
         if (OFFS && mo > 0) atomicMax(max_off, mo);
     }
+}
+
+template <bool OFFS>
+static void launch_validate(int n, int m, int64_t nnz, const int* row, const int* col, int* err, int* max_row,
+    int* max_off, short* dcol, bool need_diag, int* dpos, cudaStream_t s)
+{
+    auto k = k_validate<OFFS>;
+    const long resident = fit_grid(k, kValRows, n);
+    int R = kValRows;
+    if (nnz > (int64_t)(kValCap / kValRows) * n)
+        while (R > kValRows / 32 && ((long)n + R - 1) / R < resident) R /= 2;
+    note_launch();
+    k<<<fit_grid(k, kValRows, ((long)n + R - 1) / R), kValRows, 0, s>>>(n, m, nnz, R, row, col, err, max_row, max_off, dcol,
+        need_diag ? 1 : 0, dpos);
+    BCMGX_CHECK_LAUNCH();
 }
 
 __global__ void k_row_max(int n, const int* __restrict__ row, int* max_row)
@@ -1567,11 +1585,7 @@ int validate_csr_dev(int n, int m, int64_t nnz, const int* row, const int* col, 
     DBuf<int> st;   // error bits, longest row
     st.alloc(2, s);
     BCMGX_CUDA(cudaMemsetAsync(st.p, 0, 2 * sizeof(int), s));
-    auto k = k_validate<false>;
-    note_launch();
-    k<<<fit_grid(k, kValRows, ((long)n + kValRows - 1) / kValRows), kValRows, 0, s>>>(n, m, nnz, row, col, st.p, st.p + 1,
-        nullptr, nullptr, need_diag ? 1 : 0, nullptr);
-    BCMGX_CHECK_LAUNCH();
+    launch_validate<false>(n, m, nnz, row, col, st.p, st.p + 1, nullptr, nullptr, need_diag, nullptr, s);
     int h[2] = { 0, 0 };
     BCMGX_CUDA(cudaMemcpyAsync(h, st.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     BCMGX_CUDA(cudaStreamSynchronize(s));
@@ -2577,10 +2591,8 @@ void build_hierarchy(bcmgx_hierarchy* H, const bcmgx_csr* Ain)
         if (want16) A.dcol.alloc(A.nnz, s);
         const bool bcmg = P.preconditioner == BCMGX_PREC_BCMG;
         if (bcmg) A.dpos.alloc(A.n, s);
-        auto k = k_validate<true>;
-        note_launch();
-        k<<<fit_grid(k, kValRows, ((long)A.n + kValRows - 1) / kValRows), kValRows, 0, s>>>(A.n, A.m, A.nnz, A.row.p, A.col.p, st.p, st.p + 1, st.p + 2, want16 ? A.dcol.p : nullptr, bcmg ? 1 : 0, bcmg ? A.dpos.p : nullptr);
-        BCMGX_CHECK_LAUNCH();
+        launch_validate<true>(A.n, A.m, A.nnz, A.row.p, A.col.p, st.p, st.p + 1, st.p + 2, want16 ? A.dcol.p : nullptr,
+            bcmg, bcmg ? A.dpos.p : nullptr, s);
         int h[3] = { 0, 0, 0 };
         BCMGX_CUDA(cudaMemcpyAsync(h, st.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
         BCMGX_CUDA(cudaStreamSynchronize(s));
@@ -2745,11 +2757,7 @@ static void edge_weights_noalloc(int n, int64_t nnz, const int* row, const int* 
     int* mx = err + 1;
     note_launch();
     k_noalloc_reset<<<1, 1, 0, s>>>(minb, err, mx);
-    note_launch();
-    auto k = k_validate<false>;
-    k<<<fit_grid(k, kValRows, ((long)n + kValRows - 1) / kValRows), kValRows, 0, s>>>(n, n, nnz, row, col, err, mx, nullptr,
-        nullptr, 1, nullptr);
-    BCMGX_CHECK_LAUNCH();
+    launch_validate<false>(n, n, nnz, row, col, err, mx, nullptr, nullptr, true, nullptr, s);
     int e = read_err(err, s);
     if (e) throw Error(BCMGX_ERR_INVALID_INPUT, "input matrix: " + err_text(e));
     note_launch();

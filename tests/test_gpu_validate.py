@@ -39,8 +39,9 @@ def spoil(kind, row, col, n, r):
     return row, col
 
 
-# 255, 256, 257: a block's rows; 8192 entries: what a block stages (3 * 256 + rows of 3000 columns pass it)
-SIZES = [(1, ()), (255, ()), (256, ()), (257, ()), (3000, (5, 6, 2999)), (3000, ())]
+# 255, 256, 257: a block's rows; 8192 entries: what a block stages (3 * 256 + rows of 3000 columns pass it); 500 rows
+# of 500: longer than 32 throughout, so fewer rows a block
+SIZES = [(1, ()), (255, ()), (256, ()), (257, ()), (3000, (5, 6, 2999)), (3000, ()), (500, range(500)), (9, range(9))]
 
 
 @pytest.mark.parametrize("shift", [0, 1, 3])
@@ -64,7 +65,7 @@ def test_accepts(bx, cuda, n, dense, shift):
 
 @pytest.mark.parametrize("kind", ["first offset", "last offset", "decreasing offsets", "offset past the end",
                                   "negative column", "column too large", "not ascending", "no diagonal"])
-@pytest.mark.parametrize("n,dense", [(257, ()), (3000, (5, 6, 2999))])
+@pytest.mark.parametrize("n,dense", [(257, ()), (3000, (5, 6, 2999)), (500, range(500))])
 def test_refuses(bx, cuda, n, dense, kind):
     import torch
     row, col, val = tridiagonal(n, dense)
