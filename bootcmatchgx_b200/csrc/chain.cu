@@ -326,10 +326,21 @@ __global__ void __launch_bounds__(kChThreads) k_chain_fill(int n, int R, int S, 
     }
 }
 
-// Whether a chain of k sweeps is one launch: always from 8 sweeps up, where one launch costs less than
-// the launches it replaces for every level that fits; the usual 4 only on levels of at most 50,000
-// entries (at 105,000 entries 12.9 us against 13.6, and 16 SMs against the whole GPU beyond).
+// Whether a chain of k sweeps is one launch: from 8 sweeps up on every level that fits (chain_fits); the
+// usual 4 only on levels of at most 50,000 entries (at 105,000 entries 12.9 us against 13.6, and 16 SMs
+// against the whole GPU beyond).
 static bool chain_pays(const DevCsr& A, int k) { return k >= 8 || (k >= 2 && A.nnz <= 50000); }
+
+// Whether a block's warps have few enough slices of the level: two at most, or four on a level of at most 82,000
+// entries. A third and fourth cost a sweep more than its launch does. One cycle whose coarsest level takes 20
+// sweeps (8), launches -> cluster: 8,000 rows of 24 entries 109 -> 98 us (78 -> 74), 7,641 irregular rows 99 -> 96
+// (69 -> 67); above two slices 8,870 irregular rows would go 99 -> 105 (70 -> 71), 9,261 of 24 entries 109 -> 124
+// (79 -> 85) and 13,824 of 7 99 -> 101 (70 -> 72), but 12,167 of 7 (81,995 entries) 98 -> 96 (70 -> 69).
+static bool chain_fits(const DevCsr& A, int R, int S)
+{
+    const int slices = ceil_div(R, 32 / S);
+    return slices <= 2 * kChWarps || (slices <= kChSlices * kChWarps && A.nnz <= 82000);
+}
 
 template <typename K>
 static cudaLaunchConfig_t cluster_config(K kern, int ctas, size_t smem, cudaStream_t s, cudaLaunchAttribute* at)
@@ -390,8 +401,7 @@ static bool build_chain_t(Level& V, const T* val, bool fill, cudaStream_t s)
     P->S = S;
     P->f32 = sizeof(T) == 4;
     if (P->R > kChMaxRows) return false;
-    // more slices than the warps hold: known before anything is launched
-    if (ceil_div(P->R, 32 / S) > kChWarps * kChSlices) return false;
+    if (!chain_fits(A, P->R, S)) return false;
     P->scap = (P->R * S / 32 + 2 + 3) / 4 * 4 + 4;
     P->sptr.alloc((size_t)ctas * P->scap, s);
     P->sizes.alloc((size_t)ctas * (sizeof(ChainSizes) / sizeof(int)), s);

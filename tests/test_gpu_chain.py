@@ -183,3 +183,13 @@ def test_no_large_cluster(cuda, tmp_path):
     launches, without, with_chain = child(BCMGX_CHAIN="0"), child(LD_PRELOAD=str(lib)), child()
     assert without == launches and launches[0] == "0"
     assert int(with_chain[2]) < int(launches[2])   # the level has a chain of 16 blocks where it may
+
+
+@pytest.mark.parametrize("grid,chain", [((40, 40, 40), True), ((44, 44, 44), True), ((48, 48, 48), False)])
+def test_chain_stops_where_launches_are_faster(bx, cuda, monkeypatch, grid, chain):
+    """Coarsest levels of 8,000, 10,648 and 13,824 rows of 7 entries (two levels): the last has more than two
+    slices a warp and 93,312 entries, and keeps one launch per sweep."""
+    A = matrix(bx, ("lap7", grid))
+    _, x0, _, l0 = cycle_and_solve(bx, monkeypatch, A, "0", max_levels=2)
+    _, x1, _, l1 = cycle_and_solve(bx, monkeypatch, A, "1", max_levels=2)
+    assert (l1 < l0) == chain and np.array_equal(x0, x1)
