@@ -532,7 +532,7 @@ def run_ours(a, wl, rank, world, local_rank):
                    "fp32_rel_residual": float(nrm(b - _spmv(row, col, val, x32)) / nrm(b))},
         "spmv": {"gbs": gbs_spmv, "ms": spmv_ms, "bytes": bytes_spmv, "frac_of_peak": gbs_spmv / peak,
                  "frac_of_8TBs_nominal": gbs_spmv / 8000.0},
-        "kernels_level0": {"index_bytes": ib32, "value_bytes_fp32": vb32, "value_bytes_fp64": vb64,
+        "kernels_level0": {"index_bytes": inf32["index_bytes"][0], "value_bytes_fp32": vb32, "value_bytes_fp64": vb64,
                            "fp32_jacobi_ms": k32["jacobi"], "fp32_jacobi_gbs": gbs_jac32,
                            "fp32_jacobi_csr_equivalent_gbs": bytes_jac32_csr / (k32["jacobi"] * 1e-3) / 1e9,
                            "fp32_residual_ms": k32["residual"], "fp64_jacobi_ms": k64f["jacobi"],
@@ -752,18 +752,20 @@ def run_batch(a, rank=0, world=1, local_rank=0, steps=None, warmup=None):
                        "parallelism": f"systems round robin over {world} GPU(s), one batch graph per GPU"}}
 
 
-def block_kernel_rooflines(t, n, nnz, k):
+def block_kernel_rooflines(t, n, nnz, k, box):
     """Level-0 block kernels of the FP32-cycle multi-RHS solve (bcmgx_time_block_kernels, CUDA
     events, zero inputs): ms per launch and HBM GB/s of the algorithmic bytes (matrix once, every
     block read or written once: the gathers of X from L1/L2 are not counted) against the measured
     copy peak. The FP32 sweep reads the FP32 matrix values (8 bytes per entry with the int32
-    column), the FP64 kernels 12 bytes per entry."""
+    column), the FP64 kernels 12 bytes per entry; with box (a level in the stencil form with a table of values) the
+    sweep, the residual and the FCG product read one byte per row instead."""
     peak, kind = read_peaks()
     blk4, blk8 = 4.0 * n * k, 8.0 * n * k
-    alg = {"jacobi": 8 * nnz + 4 * (n + 1) + 4 * n + 3 * blk4,
-           "residual": 8 * nnz + 4 * (n + 1) + 3 * blk4,
-           "spmm": 12 * nnz + 4 * (n + 1) + 2 * blk8,
-           "fcg_spmm_dots": 12 * nnz + 4 * (n + 1) + 4 * blk8}
+    mat4, mat8 = 8 * nnz + 4 * (n + 1), 12 * nnz + 4 * (n + 1)
+    alg = {"jacobi": (n if box else mat4) + 4 * n + 3 * blk4,
+           "residual": (n if box else mat4) + 3 * blk4,
+           "spmm": mat8 + 2 * blk8,
+           "fcg_spmm_dots": (n if box else mat8) + 4 * blk8}
     out = {"peak_gbs": peak, "peak_kind": kind}
     for key, b in alg.items():
         ms = t[key]
@@ -773,7 +775,7 @@ def block_kernel_rooflines(t, n, nnz, k):
 
 def run_multi(a, rank=0, world=1, local_rank=0, steps=None, warmup=None, kernels=True):
     """The 27-point 100^3 Poisson matrix with 32 right-hand sides (uniform[-1,1], numpy
-    default_rng(6)) solved to 1e-8 in one block solve (CSR SpMM throughout, FP32 V-cycle) vs a
+    default_rng(6)) solved to 1e-8 in one block solve (FP32 V-cycle) vs a
     sequential loop of 32 single solves on the same hierarchy; also the block FP64-cycle solve,
     the level-0 block kernels (CUDA events, HBM GB/s of their algorithmic bytes) and the public
     SpMM call. At N > 1 rank r solves a contiguous slice of the 32 columns
@@ -844,7 +846,8 @@ def run_multi(a, rank=0, world=1, local_rank=0, steps=None, warmup=None, kernels
             res["max_rel_diff_vs_single"] = max_over_ranks(
                 max(float(torch.linalg.norm(X[:, j] - xs[j]) / torch.linalg.norm(xs[j])) for j in range(k)), world, dev)
             if kernels:
-                res["kernels_level0"] = block_kernel_rooflines(h.time_block_kernels(k, reps=20), n, nnz, k)
+                res["kernels_level0"] = block_kernel_rooflines(h.time_block_kernels(k, reps=20), n, nnz, k,
+                                                               h.info()["index_bytes"][0] < 0 and h.info()["value_codes"][0] > 0)
         h.free()
         out[prec] = res
     f32 = out["FP32"]
