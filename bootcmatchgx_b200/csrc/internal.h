@@ -74,7 +74,7 @@ bool optional_form(F&& build)
 // running, runs its prologue (reads of data that no kernel of a solve writes), then waits in
 // dep_wait() (common.cuh) for its predecessor. Only kernels that call dep_wait() before any other
 // global-memory access, and on every path, are launched this way. KIND: 0 = row kernels (plain,
-// staged, sliced), 1 = element-wise cycle kernels, 2 = FCG kernels; BCMGX_PDL is a bit mask of the
+// staged, sliced, stencil) and sweep chains (k_chain_cluster), 1 = element-wise cycle kernels, 2 = FCG kernels; BCMGX_PDL is a bit mask of the
 // kinds that get the attribute, default 1 (row kernels only). Measured on one B200 (27-point 160^3,
 // FP32 cycle): row kernels only, solve 31.4 -> 30.1 ms and one stream-launched cycle 1.19 -> 1.06 ms;
 // adding the element-wise kernels made the graph solve slower (32.3 ms), adding the FCG kernels

@@ -1988,9 +1988,8 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
     int best = default_tpr(n, A.nnz);
     float best_ms = 1e30f;
     // candidates: 1..16 threads per row, the staged kernel with 1, 2, 4 and 8 (coded negative),
-    // and the sliced and stencil kernels, whose copies of the matrix are built for their trials. The sliced
-    // copy goes before the stencil's comes, so that the trials never hold both (on 7-point 256^3
-    // they would be the peak of the set-up); the caller builds it again when it wins.
+    // and the sliced and stencil kernels, whose copies of the matrix are built for their trials and kept if they
+    // win. The sliced copy makes room for the stencil's where memory is short (the caller builds it again when it wins).
     bool room = true;
     for (int t : {1, 2, 4, 8, 16, -1, -2, -4, -8, kSlicedCode, kStencilCode}) {
         if (t == kSlicedCode) {
@@ -1999,8 +1998,13 @@ int autotune_tpr(Level& V, bool f32, bool need64, cudaStream_t s)
         }
         if (t == kStencilCode) {
             if (!like) continue;
-            release_sliced(A);
-            room = optional_form([&] { build_stencil(A, need64, s); });
+            auto build = [&] { build_stencil(A, need64, s); };
+            room = optional_form(build);
+            if (!room) {
+                release_stencil(A);
+                release_sliced(A);
+                room = optional_form(build);
+            }
             if (!room || !A.st_form.p) continue;
         }
         const bool own = t == kSlicedCode || t == kStencilCode;
