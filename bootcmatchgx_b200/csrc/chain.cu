@@ -36,9 +36,13 @@ constexpr int kChMaxRows = 2047;         // rows of a block at most (11 bits of 
 constexpr int kChHalo = 8192;            // halo slots and push entries of a block at most
 
 // Per block: sizes, and its arrays at rank * (cap) of the plan's buffers.
-struct ChainSizes {
-    int entries, halo, push, slices, width;   // width: steps of the widest slice
-    int need[kChCtas];                        // halo slots by the block that owns their rows
+struct alignas(16) ChainSizes {
+    int entries, halo, push, slices;
+    int width;   // steps of the widest slice
+};
+// and after them (while the plan is made): every block's halo slots by the block that owns their rows
+struct ChainNeeds {
+    int of[kChCtas];
 };
 
 template <typename T>
@@ -238,13 +242,13 @@ struct ChainHalo {
 // The plan's sizes, a block of the grid for each of the cluster's: its slices' widths (sptr) and its halo.
 // Neither this nor k_chain_fill is a cluster: where none of the wanted size can run, set-up goes on without.
 __global__ void __launch_bounds__(kChThreads) k_chain_sizes(int n, int R, int S, int scap, const int* __restrict__ row,
-    const int* __restrict__ col, int* __restrict__ sptr, ChainSizes* sizes)
+    const int* __restrict__ col, int* __restrict__ sptr, ChainSizes* sizes, ChainNeeds* needs)
 {
     __shared__ ChainHalo halo;
     const int rank = blockIdx.x, tid = threadIdx.x;
     const int r0 = rank * R, nr = max(0, min(R, n - r0)), rs = 32 / S, slices = (nr + rs - 1) / rs;
     const int H = halo.build(n, R, rank, row, col);
-    if (tid < (int)gridDim.x) sizes[rank].need[tid] = halo.slots_below((tid + 1) * R, n, H) - halo.slots_below(tid * R, n, H);
+    if (tid < (int)gridDim.x) needs[rank].of[tid] = halo.slots_below((tid + 1) * R, n, H) - halo.slots_below(tid * R, n, H);
     if (tid < 32) {
         int at = 0, widest = 0;
         for (int t0 = 0; t0 < slices; t0 += 32) {
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(kChThreads) k_chain_sizes(int n, int R, int S,
 template <typename T>
 __global__ void __launch_bounds__(kChThreads) k_chain_fill(int n, int R, int S, int ecap, int pcap, int scap,
     const int* __restrict__ row, const int* __restrict__ col, const T* __restrict__ val, const int* __restrict__ sptr,
-    T* __restrict__ pval, unsigned short* __restrict__ pidx, unsigned* __restrict__ push, ChainSizes* sizes)
+    T* __restrict__ pval, unsigned short* __restrict__ pidx, unsigned* __restrict__ push, ChainSizes* sizes, const ChainNeeds* __restrict__ needs)
 {
     __shared__ ChainHalo halo;
     __shared__ int at[kChCtas];
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(kChThreads) k_chain_fill(int n, int R, int S, 
         int o = 0, all = 0;
         for (int c = 0; c < (int)gridDim.x; c++) {
             if (c == rank) o = all;
-            all += sizes[c].need[tid];
+            all += needs[c].of[tid];
         }
         at[tid] = o - halo.slots_below(tid * R, n, H);
         if (tid == rank) sizes[rank].push = all;
@@ -404,18 +408,22 @@ static bool build_chain_t(Level& V, const T* val, bool fill, cudaStream_t s)
     if (!chain_fits(A, P->R, S)) return false;
     P->scap = (P->R * S / 32 + 2 + 3) / 4 * 4 + 4;
     P->sptr.alloc((size_t)ctas * P->scap, s);
-    P->sizes.alloc((size_t)ctas * (sizeof(ChainSizes) / sizeof(int)), s);
+    const size_t sizes_bytes = (size_t)ctas * sizeof(ChainSizes);
+    P->sizes.alloc((sizes_bytes + (size_t)ctas * sizeof(ChainNeeds)) / sizeof(int), s);
     ChainSizes* const sizes = (ChainSizes*)P->sizes.p;
+    ChainNeeds* const needs = (ChainNeeds*)(sizes + ctas);
     note_launch();
-    k_chain_sizes<<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->scap, A.row.p, A.col.p, P->sptr.p, sizes);
+    k_chain_sizes<<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->scap, A.row.p, A.col.p, P->sptr.p, sizes, needs);
     BCMGX_CHECK_LAUNCH();
-    ChainSizes z[kChCtas];
-    BCMGX_CUDA(cudaMemcpyAsync(z, sizes, sizeof(ChainSizes) * ctas, cudaMemcpyDeviceToHost, s));
+    std::vector<unsigned char> host(sizes_bytes + (size_t)ctas * sizeof(ChainNeeds));
+    BCMGX_CUDA(cudaMemcpyAsync(host.data(), sizes, host.size(), cudaMemcpyDeviceToHost, s));
     BCMGX_CUDA(cudaStreamSynchronize(s));
+    const ChainSizes* z = (const ChainSizes*)host.data();
+    const ChainNeeds* zn = (const ChainNeeds*)(z + ctas);
     int E = 0, H = 0, N = 0, W = 0;
     for (int c = 0; c < ctas; c++) {
         int push = 0;
-        for (int b = 0; b < ctas; b++) push += z[b].need[c];
+        for (int b = 0; b < ctas; b++) push += zn[b].of[c];
         if (z[c].entries > kChSmem / (int)(sizeof(T) + 2) || z[c].halo > kChHalo || push > kChHalo) return false;
         P->pcap = std::max(P->pcap, push);
         E = std::max(E, z[c].entries);
@@ -460,7 +468,7 @@ static bool build_chain_t(Level& V, const T* val, bool fill, cudaStream_t s)
     P->push.alloc((size_t)ctas * P->pcap, s);
     note_launch();
     k_chain_fill<T><<<ctas, kChThreads, 0, s>>>(n, P->R, S, P->ecap, P->pcap, P->scap, A.row.p, A.col.p, val, P->sptr.p,
-        (T*)P->val.p, P->idx.p, P->push.p, sizes);
+        (T*)P->val.p, P->idx.p, P->push.p, sizes, needs);
     BCMGX_CHECK_LAUNCH();
     V.chain = std::move(P);
     return true;
